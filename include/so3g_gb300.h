@@ -201,7 +201,8 @@ int64_t so3g_launch_count(void);
  * the previous value (default 30,000,000; no counterpart in the reference,
  * whose pointing has one form).  Smaller calls take the per-sample float32
  * tier, whose fixed cost per call is lower; results agree within the mixed
- * pointing's tolerance either way.  Process-wide; negative values count as
+ * pointing's tolerance either way.  The chunked certified kernels (the same
+ * results as the general ones) take calls of a tenth of it.  Process-wide; negative values count as
  * 0 (every eligible call chunked). */
 int64_t so3g_set_chunked_min_samples(int64_t n);
 

@@ -36,7 +36,8 @@ def set_chunked_min_samples(n):
     """Sets the smallest call (detectors x samples, whole detectors) that
     takes the chunked mixed-pointing kernels; returns the previous value
     (default 3e7: smaller calls take the per-sample float32 tier, whose
-    fixed cost per call is lower).  Process-wide."""
+    fixed cost per call is lower).  The chunked certified kernels take calls
+    of a tenth of it.  Process-wide."""
     from . import _abi
     return int(_abi.lib().so3g_set_chunked_min_samples(int(n)))
 

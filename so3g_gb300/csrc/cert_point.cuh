@@ -1,0 +1,874 @@
+// cert_point.cuh -- chunked pointing for the certified mode
+// (SO3G_POINTING_CERTIFIED) with nearest-neighbour pixelizors: the pointing
+// of 64 consecutive samples of a detector from one polynomial model whose
+// results are the float64 path's, bit for bit.
+//
+// The certified double-float pointing (fastpoint.cuh) costs ~900
+// instructions a sample, nearly all of them in the quaternion product and
+// the spin factors, and the projection kernels are bound by instruction
+// issue.  Along a scan the pointing is smooth, so here it is evaluated once
+// per 64-sample chunk, at the chunk's middle, and expanded about it: per
+// sample a float32 cubic for each pixel coordinate and, for each spin
+// factor, an exactly representable float32 part plus a float32 correction.
+// Both carry a bound on their distance from the reference's float64 value;
+// a sample whose pixel or whose float32 rounding of a spin factor is not
+// certain goes to the per-sample certified path (and from there, if need
+// be, to the float64 path), so every result is that of the exact path.
+//
+// The boresight of a chunk is modelled by a polynomial Q(u) (u = (t - tm) /
+// 64, tm its middle sample): the quartic through five of its samples where
+// that fits every sample to ~1e-13, else (time stamps and encoders jitter)
+// the quadratic through its first, middle and last sample, with the
+// residual of each sample kept as a small rotation rho, q(t) = Q (1 + rho),
+// in 3 x 16 bits.
+//
+// With A(u) = Q(u) q_det, alpha = a + i d and beta = c + i b are polynomials
+// in u, alpha = alpha_0 (1 + z_1 u + z_2 u^2 + ...), and so are, to the order
+// kept, their logarithms la(u) = log(alpha / alpha_0) and lb(u).  In these
+// terms (Pointer<C>::GetCoords, src/Projection.cxx:337-507)
+//   CAR   lon = arg(alpha) - arg(beta),   atanh(sin lat) = ln|alpha / beta|,
+//         spin factors P exp(2 i (arg(alpha) + arg(beta)))
+//   zenithal   Y - i X = 2 alpha conj(beta) g(|alpha|^2),   g(n) = 1 (SIN),
+//         1 / (2n - 1) (TAN), 1 / sqrt(n) (ZEA),
+//         spin factors P exp(4 i arg(alpha)).
+// The spin factors are expanded to u^4, their u^1 coefficient in
+// double-float, the pixel coordinates to u^3; the terms left out are
+// bounded by the majorant series of the logarithms and the exponential
+// (cx_tail5; ~1e-13 on the 1 deg/s scans of the workloads).  The residual
+// turns the spin factors' phase phi by grad(phi) . rho, the gradient a linear
+// function of u per chunk and detector, and moves the pixel by at most
+// 2 |rho| / cos(lat), which goes into the pixel's bound.
+#pragma once
+
+#include "host.h"
+
+namespace so3g {
+
+namespace {
+
+constexpr int kCxLen = 64;            // samples per chunk
+constexpr int kCxMid = kCxLen / 2;
+constexpr int kCxGroup = 32;          // chunks of a warp's group, one per lane
+// A boresight whose residuals exceed this in more than a quarter of its
+// chunks (pointing noise of ~0.03") is not taken: the call's general kernel
+// is faster than sending most samples to the per-sample path (200 det x 500k,
+// to_map: noise of 1e-8 per quaternion component 1.26 ms against 2.83, 1e-7
+// 2.4 on a CAR map and 6.8 on a fast HEALPix scan against 2.8 and 3.4, 1e-6
+// 5.7 against 2.8).
+constexpr float kCxRough = 6e-7f;
+
+// Classes of coordinate systems the models are compiled for.
+enum { CX_CAR = 0, CX_ZEN = 1 };
+
+// The boresight model of one chunk, Q = q + u a1 + u^2 a2 + u^3 a3 + u^4 a4.
+struct __align__(16) CxBore {
+    float4 q_hi, q_lo, a1_hi, a1_lo;   // double-float
+    float4 a2, a3, a4;
+    float e;               // max |q(t) - Q|
+    float eta;             // max ||q(t)|^2 - 1|
+    float lsb;             // residuals' unit; 0: none kept (e is negligible)
+    float pad;
+};
+
+// The boresight models of a call: per chunk, and the residuals per sample.
+struct CxModel {
+    const CxBore *bore;
+    const short4 *resid;
+};
+
+// Per (detector, chunk), nine 16-byte words (an odd number: neighbouring
+// chunks' slots start on different shared-memory banks):
+//   0: x0 x1 x2 x3   1: y0 y1 y2 y3   2: hx hy e -   3: xb yb mid flag
+//   4: f0 f1 l0 l1   5: a2 a3 a4 g0x  6: f0 f1 l0 l1   7: a2 a3 a4 g0y
+//   8: g0z g1x g1y g1z
+// With k = t - mid: x = xb + 1/2 + x0 + k (x1 + k (x2 + k x3)) (xb less the
+// bits of kCxMagic); a spin factor is
+// (f0 + k f1), exact in float32, plus the correction l0 + k (l1 + k (a2 + k
+// (a3 + k a4))), within e, plus (flag) the residual's turn.  hx, hy: 1/2 -
+// bounds (pixels; -1: not modelled).  HEALPix: x is the longitude and y
+// sin(lat), with xb = yb = 0 and hx, hy their error bounds (hx < 0: not
+// modelled).  g0 + k g1: the gradient of phi, per residual unit.
+constexpr int kCxWords = 9;
+// 1.5 x 2^23: x + kCxMagic is x rounded to the nearest integer (|x| < 2^21),
+// its low bits that integer -- one addition instead of a floor and a
+// conversion on the slow conversion pipe.
+constexpr float kCxMagic = 12582912.f;
+constexpr int kCxMagicBits = 0x4b400000;
+
+// Middle sample of chunk j (samples [64 j, 64 j + 64)); the last chunk's is
+// moved back so that its model's samples mid - 32 .. mid + 32 exist.
+__device__ __forceinline__ int cx_mid(int j, int n_time) {
+    return min(j * kCxLen, n_time - 1 - kCxLen) + kCxMid;
+}
+
+// The chunks' boresight models and residuals, 16 threads per chunk (one per
+// quaternion component and quarter of its samples), in double-float
+// arithmetic (the float64 pipe would take ~0.1 ms per million samples).
+__global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time, int n_chunks,
+                                                 CxBore *out, short4 *resid,
+                                                 unsigned *rough) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int chunk = i >> 4, j = min(chunk, n_chunks - 1), comp = i & 3, part = (i >> 2) & 3;
+    const int base = cx_mid(j, n_time) - kCxMid;
+    const double *b = bore + 4LL * base + comp;
+    bool bad = false;   // a value df_split does not take (or NaN, infinity)
+    dfl q[5];
+#pragma unroll
+    for (int k = 0; k < 5; k++) bad |= !df_split(__ldg(b + kCxLen * k), q[k]);
+    // Central differences about the middle, odd and even.
+    const dfl o1 = df_sub(q[3], q[1]), o2 = df_sub(q[4], q[0]);
+    const dfl two2 = df_mulf(q[2], 2.f);
+    const dfl e1 = df_sub(df_add(q[1], q[3]), two2), e2 = df_sub(df_add(q[0], q[4]), two2);
+    // Quartic, samples h = 1/4 apart: a1 = (8 o1 - o2) / (12 h), a2 = (16 e1 -
+    // e2) / (24 h^2), a3 = (o2 - 2 o1) / (12 h^3), a4 = (e2 - 4 e1) / (24 h^4).
+    const dfl third{0.33333334f, -9.934108e-09f};
+    const dfl a1 = df_mul(df_sub(df_mulf(o1, 8.f), o2), third);
+    const dfl a2 = df_mul(df_mulf(df_sub(df_mulf(e1, 16.f), e2), 2.f), third);
+    const float a3 = df_sub(o2, df_mulf(o1, 2.f)).hi * (16.f / 3.f);
+    const float a4 = df_sub(e2, df_mulf(e1, 4.f)).hi * (32.f / 3.f);
+    // Quadratic through the first, middle and last sample.
+    const dfl b1 = o2, b2 = df_mulf(e2, 2.f);
+    const int k0 = j * kCxLen - base;                        // first own sample
+    const int k1 = min(kCxLen - 1 + k0, n_time - 1 - base);  // last own sample
+    float r4 = 0.f, r2 = 0.f, eta = 0.f;
+    for (int n = 0; n < kCxLen / 4; n++) {   // (the same count in every lane)
+        const int k = min(k0 + part * (kCxLen / 4) + n, k1);
+        dfl v;
+        bad |= !df_split(__ldg(b + 4 * k), v);
+        const float u = (float)(k - kCxMid) * (1.f / kCxLen);
+        const dfl d = df_sub(v, q[2]);
+        const dfl p4 =
+            df_mulf(df_add(a1, df_mulf(df_add(a2, dfl{u * fmaf(u, a4, a3), 0.f}), u)), u);
+        const dfl p2 = df_mulf(df_add(b1, df_mulf(b2, u)), u);
+        r4 = fmaxf(r4, fabsf(df_sub(d, p4).hi));   // (fmaxf drops NaN: only a bad
+        r2 = fmaxf(r2, fabsf(df_sub(d, p2).hi));   // value makes one)
+        dfl s = df_mul(v, v);
+        s = df_add(s, dfl{__shfl_xor_sync(kFull, s.hi, 1), __shfl_xor_sync(kFull, s.lo, 1)});
+        s = df_add(s, dfl{__shfl_xor_sync(kFull, s.hi, 2), __shfl_xor_sync(kFull, s.lo, 2)});
+        eta = fmaxf(eta, fabsf(df_sub(s, dfl{1.f, 0.f}).hi));
+    }
+    bad = __any_sync(kFull, bad);   // (the warp's other chunk as well)
+    auto max_parts = [](float x) {
+        x = fmaxf(x, __shfl_xor_sync(kFull, x, 4));
+        return fmaxf(x, __shfl_xor_sync(kFull, x, 8));
+    };
+    auto sum4 = [](float x) {
+        x += __shfl_xor_sync(kFull, x, 1);
+        return x + __shfl_xor_sync(kFull, x, 2);
+    };
+    r4 = max_parts(r4);
+    r2 = max_parts(r2);
+    eta = max_parts(eta);
+    // 1e-13: the double-float roundings.
+    const float E4 = sqrtf(sum4(r4 * r4)) * 1.00001f + 1e-13f;
+    const float E2 = sqrtf(sum4(r2 * r2)) * 1.00001f + 1e-13f;
+    const bool quad = !(E4 < 2.5e-13f);
+    const float lsb = quad && !bad ? E2 * (1.f / 32000.f) : 0.f;
+    if (chunk < n_chunks && part == 0) {
+        float *o = reinterpret_cast<float *>(out + j);
+        o[comp] = q[2].hi;
+        o[4 + comp] = q[2].lo;
+        o[8 + comp] = quad ? b1.hi : a1.hi;
+        o[12 + comp] = quad ? b1.lo : a1.lo;
+        o[16 + comp] = quad ? b2.hi : a2.hi;
+        o[20 + comp] = quad ? 0.f : a3;
+        o[24 + comp] = quad ? 0.f : a4;
+        if (comp == 0) {
+            if (bad || (quad && !(E2 < kCxRough))) atomicAdd(rough, 1u);
+            out[j].e = bad ? 1.f : (quad ? E2 : E4);
+            out[j].eta = bad ? 1.f : eta * 1.00001f + 1e-14f;
+            out[j].lsb = lsb;
+        }
+    }
+    // Residuals: rho = conj(Q) (q - Q), in units of lsb.
+    if (!__any_sync(kFull, lsb > 0.f)) return;
+    const float inv = lsb > 0.f ? 1.f / lsb : 0.f;
+    const int lane0 = threadIdx.x & 28;
+    for (int n = 0; n < kCxLen / 4; n++) {
+        const int k = k0 + part * (kCxLen / 4) + n, kc = min(k, k1);
+        dfl v;
+        df_split(__ldg(b + 4 * kc), v);
+        const float u = (float)(kc - kCxMid) * (1.f / kCxLen);
+        const dfl p2 = df_mulf(df_add(b1, df_mulf(b2, u)), u);
+        const float r = df_sub(df_sub(v, q[2]), p2).hi * inv, g = v.hi;
+        float rr[4], qq[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            rr[c] = __shfl_sync(kFull, r, lane0 + c);
+            qq[c] = __shfl_sync(kFull, g, lane0 + c);
+        }
+        if (comp == (k & 3) && k <= k1 && chunk < n_chunks && inv > 0.f) {
+            const float x = qq[0] * rr[1] - qq[1] * rr[0] - qq[2] * rr[3] + qq[3] * rr[2];
+            const float y = qq[0] * rr[2] + qq[1] * rr[3] - qq[2] * rr[0] - qq[3] * rr[1];
+            const float z = qq[0] * rr[3] - qq[1] * rr[2] + qq[2] * rr[1] - qq[3] * rr[0];
+            resid[base + k] = make_short4((short)__float2int_rn(x), (short)__float2int_rn(y),
+                                          (short)__float2int_rn(z), 0);
+        }
+    }
+}
+
+// Complex float32.
+struct cf {
+    float r, i;
+};
+__device__ __forceinline__ cf operator+(cf a, cf b) { return cf{a.r + b.r, a.i + b.i}; }
+__device__ __forceinline__ cf operator-(cf a, cf b) { return cf{a.r - b.r, a.i - b.i}; }
+__device__ __forceinline__ cf operator*(float s, cf a) { return cf{s * a.r, s * a.i}; }
+__device__ __forceinline__ cf operator*(cf a, cf b) {
+    return cf{fmaf(a.r, b.r, -a.i * b.i), fmaf(a.r, b.i, a.i * b.r)};
+}
+__device__ __forceinline__ float cf_abs(cf a) {
+    const float n = fmaf(a.r, a.r, a.i * a.i);
+    return n > 1e-36f ? 1.000001f * n * rsqrtf(n) : 1e-18f;
+}
+
+__device__ __forceinline__ void cx_qmul(const float4 &p, const float (&q)[4], float (&r)[4]) {
+    r[0] = p.x * q[0] - p.y * q[1] - p.z * q[2] - p.w * q[3];
+    r[1] = p.x * q[1] + p.y * q[0] + p.z * q[3] - p.w * q[2];
+    r[2] = p.x * q[2] - p.y * q[3] + p.z * q[0] + p.w * q[1];
+    r[3] = p.x * q[3] + p.y * q[2] - p.z * q[1] + p.w * q[0];
+}
+
+// log(1 + z1 u + z2 u^2 + z3 u^3 + z4 u^4) to u^4.
+struct CxLog {
+    cf l1, l2, l3, l4;
+};
+__device__ __forceinline__ CxLog cx_log(cf z1, cf z2, cf z3, cf z4) {
+    const cf s = z1 * z1;
+    CxLog o;
+    o.l1 = z1;
+    o.l2 = z2 - 0.5f * s;
+    o.l3 = z3 - z1 * z2 + (1.f / 3.f) * (s * z1);
+    o.l4 = z4 - z1 * z3 - 0.5f * (z2 * z2) + s * z2 - 0.25f * (s * s);
+    return o;
+}
+
+// For nonnegative c1..c4 (a polynomial's coefficients at the chunk's end),
+// the terms of order >= 5 of X^2, X^3 and X^4, X = c1 t + ... + c4 t^4 at t =
+// 1 (bounds: the differences' float32 cancellation is in the 1e-15).
+struct CxTail {
+    float t2, t3, t4, X;
+};
+__device__ __forceinline__ CxTail cx_tail(float c1, float c2, float c3, float c4) {
+    CxTail o;
+    const float X = c1 + c2 + c3 + c4, r = c2 + c3 + c4;
+    o.X = X;
+    o.t2 = 2.f * (c1 * c4 + c2 * (c3 + c4) + c3 * c4) + c3 * c3 + c4 * c4;
+    // X^3 - c1^3 - 3 c1^2 c2 and X^4 - c1^4, with X = c1 + r.
+    o.t3 = 3.f * c1 * c1 * (c3 + c4) + 3.f * c1 * r * r + r * r * r;
+    o.t4 = r * (4.f * c1 * c1 * c1 + r * (6.f * c1 * c1 + r * (4.f * c1 + r)));
+    return o;
+}
+// Terms of order >= 5 left out of the logarithm of 1 + X (n-th power / n).
+__device__ __forceinline__ float cx_tail_log(const CxTail &t) {
+    const float x2 = t.X * t.X;
+    return 0.5f * t.t2 + (1.f / 3.f) * t.t3 + 0.25f * t.t4 + 0.25f * x2 * x2 * t.X;
+}
+// ... and of the exponential of X (n-th power / n!).
+__device__ __forceinline__ float cx_tail_exp(const CxTail &t) {
+    const float x2 = t.X * t.X;
+    return 0.5f * t.t2 + (1.f / 6.f) * t.t3 + (1.f / 24.f) * t.t4 + (1.f / 100.f) * x2 * x2 * t.X;
+}
+
+// Gradient of phi with respect to a rotation rho of the boresight (q (1 +
+// rho) q_det), at A = q q_det.  In the detector's frame (rho' = conj(q_det)
+// rho q_det = (x, y, z)): d log(alpha) = i z - (y + i x) conj(beta) / alpha,
+// d log(beta) = i z + (y + i x) conj(alpha) / beta, so dphi = 4 z + 2 Im((y
+// + i x) kappa), kappa = (|alpha|^2 - |beta|^2) / (alpha beta) (CAR) or -2
+// conj(beta) / alpha (zenithal).  Returns |kappa|.
+template <int CL>
+__device__ __forceinline__ float cx_gradient(const float (&A)[4], const float (&d)[4],
+                                             float (&g)[3]) {
+    const cf al{A[0], A[3]}, be{A[2], A[1]};
+    cf k;
+    if (CL == CX_CAR) {
+        const cf v = al * be;
+        const float z = (al.r * al.r + al.i * al.i) - (be.r * be.r + be.i * be.i);
+        const float f = z * rcp_approx(v.r * v.r + v.i * v.i);
+        k = cf{v.r * f, -v.i * f};
+    } else {
+        const cf v = al * be;
+        const float f = -2.f * rcp_approx(al.r * al.r + al.i * al.i);
+        k = cf{v.r * f, -v.i * f};
+    }
+    // To the boresight's frame: q_det g' conj(q_det).
+    const float x = 2.f * k.r, y = 2.f * k.i, z = 4.f;
+    const float tx = 2.f * (d[2] * z - d[3] * y), ty = 2.f * (d[3] * x - d[1] * z),
+                tz = 2.f * (d[1] * y - d[2] * x);
+    g[0] = x + d[0] * tx + d[2] * tz - d[3] * ty;
+    g[1] = y + d[0] * ty + d[3] * tx - d[1] * tz;
+    g[2] = z + d[0] * tz + d[1] * ty - d[2] * tx;
+    return cf_abs(k);
+}
+
+// The model of chunk j for a detector (double-float qd), into w (kCxWords
+// words).
+template <int CL, bool HP, int NC, class Args>
+__device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int coord, int j,
+                                         int n_time, const dfl (&qd)[4], float Pr, float4 *w) {
+    constexpr bool SPIN = NC > 1;
+    constexpr float u = kU;
+    const int mid = cx_mid(j, n_time);
+    w[2] = make_float4(-1.f, -1.f, 0.f, 0.f);
+    w[3] = make_float4(0.f, 0.f, __int_as_float(mid), 0.f);
+    const CxBore &cb = cxb[j];
+    const float E = __ldg(&cb.e), lsb = __ldg(&cb.lsb);
+    if (!(E < 1e-6f)) return;
+    // The middle sample: its coordinates X0, Y0 (HEALPix: longitude and
+    // sin(lat)) and spin quantities, certified double-float.
+    dfl qa, qb, qc, qe, X0, Y0, Nc, Ns, D;
+    {
+        const float4 h = __ldg(&cb.q_hi), l = __ldg(&cb.q_lo);
+        const dfl q[4] = {{h.x, l.x}, {h.y, l.y}, {h.z, l.z}, {h.w, l.w}};
+        df_qmul(q, qd, qa, qb, qc, qe);
+    }
+    if constexpr (HP) {
+        Y0 = df_dot<4>({qa, qb, qc, qe}, {qa, df_neg(qb), df_neg(qc), qe});
+        if (!(fabsf(Y0.hi) < 0.99f) ||
+            !fast_lon_spin(a.ft, a.fc, qa, qb, qc, qe, Y0, X0, Nc, Ns, D))
+            return;
+    } else if constexpr (CL == CX_CAR) {
+        if (!fast_car(a.ft, a.fc, qa, qb, qc, qe, X0, Y0, Nc, Ns, D)) return;
+    } else {
+        dfl n, p, v;
+        fast_zen_nuv(qa, qb, qc, qe, n, p, v);
+        bool ok;
+        if (coord == SO3G_COORD_TAN)
+            ok = fast_zen_xy<SO3G_COORD_TAN>(a.ft, a.fc, qb, qc, n, p, v, X0, Y0);
+        else if (coord == SO3G_COORD_ZEA)
+            ok = fast_zen_xy<SO3G_COORD_ZEA>(a.ft, a.fc, qb, qc, n, p, v, X0, Y0);
+        else
+            ok = fast_zen_xy<SO3G_COORD_SIN>(a.ft, a.fc, qb, qc, n, p, v, X0, Y0);
+        if (!ok) return;
+        fast_zen_spin(qa, qe, n, Nc, Ns, D);
+    }
+    // The float32 polynomials of alpha and beta.
+    const float d32[4] = {qd[0].hi, qd[1].hi, qd[2].hi, qd[3].hi};
+    const float A[4] = {qa.hi, qb.hi, qc.hi, qe.hi};
+    float A1[4], A2[4], A3[4], A4[4];
+    cx_qmul(__ldg(&cb.a1_hi), d32, A1);
+    cx_qmul(__ldg(&cb.a2), d32, A2);
+    cx_qmul(__ldg(&cb.a3), d32, A3);
+    cx_qmul(__ldg(&cb.a4), d32, A4);
+    const float al2 = A[0] * A[0] + A[3] * A[3], be2 = A[1] * A[1] + A[2] * A[2];
+    const float nq2 = d32[0] * d32[0] + d32[1] * d32[1] + d32[2] * d32[2] + d32[3] * d32[3];
+    if (!(fabsf(al2 + be2 - 1.f) < 1e-3f && fabsf(nq2 - 1.f) < 1e-3f && al2 > 0.004f)) return;
+    const float ia = rcp_approx(al2);
+    const cf inv_a{A[0] * ia, -A[3] * ia};
+    const CxLog la = cx_log(cf{A1[0], A1[3]} * inv_a, cf{A2[0], A2[3]} * inv_a,
+                            cf{A3[0], A3[3]} * inv_a, cf{A4[0], A4[3]} * inv_a);
+    // |z_n| / 2^n: sizes at the chunk's end.
+    const float ra = rsqrtf(al2) * 1.0001f;
+    const CxTail ta = cx_tail(0.5f * ra * cf_abs(cf{A1[0], A1[3]}), 0.25f * ra * cf_abs(cf{A2[0], A2[3]}),
+                              0.125f * ra * cf_abs(cf{A3[0], A3[3]}),
+                              0.0625f * ra * cf_abs(cf{A4[0], A4[3]}));
+    if (!(ta.X < 0.05f)) return;
+    float tail = cx_tail_log(ta);    // logarithms' terms of order >= 5
+    float phi1, phi2, phi3, phi4;    // phase of the spin factors
+    float cx1, cx2, cx3, cy1, cy2, cy3;   // X, Y: cubic in u
+    float tx, ty;                    // their terms of order >= 4
+    float rx, ry;                    // X, Y per unit of residual
+    float lutx = 0.f, luty = 0.f;    // the tables' errors at both ends
+    float zz;                        // |z1|^2 of alpha and beta
+    float gerr;                      // gradient of phi: error of its linear form
+    if constexpr (CL == CX_CAR) {
+        if (!(be2 > 0.004f)) return;
+        const float ib = rcp_approx(be2);
+        const cf inv_b{A[2] * ib, -A[1] * ib};
+        const CxLog lb = cx_log(cf{A1[2], A1[1]} * inv_b, cf{A2[2], A2[1]} * inv_b,
+                                cf{A3[2], A3[1]} * inv_b, cf{A4[2], A4[1]} * inv_b);
+        const float rb = rsqrtf(be2) * 1.0001f;
+        const CxTail tb =
+            cx_tail(0.5f * rb * cf_abs(cf{A1[2], A1[1]}), 0.25f * rb * cf_abs(cf{A2[2], A2[1]}),
+                    0.125f * rb * cf_abs(cf{A3[2], A3[1]}), 0.0625f * rb * cf_abs(cf{A4[2], A4[1]}));
+        if (!(tb.X < 0.05f)) return;
+        tail += cx_tail_log(tb);
+        phi1 = 2.f * (la.l1.i + lb.l1.i);
+        phi2 = 2.f * (la.l2.i + lb.l2.i);
+        phi3 = 2.f * (la.l3.i + lb.l3.i);
+        phi4 = 2.f * (la.l4.i + lb.l4.i);
+        zz = 4.f * (ta.X * ta.X + tb.X * tb.X);
+        cx1 = la.l1.i - lb.l1.i;
+        cx2 = la.l2.i - lb.l2.i;
+        cx3 = la.l3.i - lb.l3.i;
+        tx = 0.0625f * fabsf(la.l4.i - lb.l4.i) + tail;
+        // Latitude from m = ln|alpha / beta| - its value at the middle: with
+        // S, C = sin, cos of the latitude, dlat/dm = C, dS/dm = C^2.
+        const float m1 = la.l1.r - lb.l1.r, m2 = la.l2.r - lb.l2.r, m3 = la.l3.r - lb.l3.r;
+        const float S = al2 - be2, C2 = 4.f * al2 * be2, C = C2 * rsqrtf(C2);
+        const float mu1 = 0.5f * fabsf(m1), mu2 = 0.25f * fabsf(m2), mu3 = 0.125f * fabsf(m3),
+                    mu4 = 0.0625f * fabsf(la.l4.r - lb.l4.r) + tail;
+        const float mu = mu1 + mu2 + mu3 + mu4;
+        // kappa = S / v, |v| = C / 2: |kappa''| / 8 with |(1/v)'| <= |z1a| +
+        // |z1b|, |S'| <= C^2 |m1|, |S''| <= 2 C^2 (m1^2 + |m2|).
+        const float zs1 = 2.f * (ta.X + tb.X);
+        gerr = 0.3f * fabsf(S) * rsqrtf(C2) * zs1 * zs1 +
+               C * fabsf(m1) * (0.6f * zs1 + 0.6f * fabsf(m1)) + 0.6f * C * fabsf(m2);
+        // Order >= 4: m's own, those of m^2 / 2 and m^3 / 6 (derivatives at
+        // most 2 and 4), and the fourth derivative's (at most 10).
+        ty = mu4 + (2.f * mu1 * (mu3 + mu4) + (mu2 + mu3 + mu4) * (mu2 + mu3 + mu4)) +
+             2.f * (mu * mu * mu - mu1 * mu1 * mu1) + 0.5f * mu * mu * mu * mu + 1e-12f;
+        if constexpr (HP) {
+            cy1 = C2 * m1;
+            cy2 = C2 * (m2 - S * m1 * m1);
+            cy3 = C2 * (m3 - 2.f * S * m1 * m2 - (C2 - 2.f * S * S) * (1.f / 3.f) * m1 * m1 * m1);
+        } else {
+            cy1 = C * m1;
+            cy2 = C * (m2 - 0.5f * S * m1 * m1);
+            cy3 = C * (m3 - S * m1 * m2 + (S * S - C2) * (1.f / 6.f) * m1 * m1 * m1);
+        }
+        rx = 1.05f * ra * rb;
+        ry = 2.1f;
+        // h^2/8 max|f''| of the tables: ATAN2 3.0e-10, ASIN 4.66e-10 S (1 -
+        // S^2)^-3/2 (at an S beyond the chunk's); the middle's and the sample's.
+        const float zs = fminf(fabsf(S) + 1.1f * C * mu, 0.9985f);
+        const float rs = rsqrtf(1.f - zs * zs);
+        lutx = 2.f * 3.1e-10f;
+        luty = (HP ? 1.f : 2.f) * 4.7e-10f * zs * rs * rs * rs;
+        // The longitude stays inside (-pi, pi) over the chunk (a HEALPix pixel
+        // takes it modulo 2 pi).
+        if (!HP && !(fabsf(X0.hi) + 1.05f * (ta.X + tb.X) + rx * E + 1e-6f < 3.1415f)) return;
+    } else {
+        phi1 = 4.f * la.l1.i;
+        phi2 = 4.f * la.l2.i;
+        phi3 = 4.f * la.l3.i;
+        phi4 = 4.f * la.l4.i;
+        zz = 4.f * ta.X * ta.X;
+        if (!(al2 > 0.25f)) return;
+        // kappa = -2 conj(beta) / alpha: |kappa''| / 8.
+        gerr = 0.6f * ra * (cf_abs(cf{A2[2], A2[1]}) + 2.f * ta.X * cf_abs(cf{A1[2], A1[1]}) +
+                            4.f * ta.X * ta.X);
+        // Y - i X = 2 g(n_0) alpha_0 e(u) conj(beta), e = (alpha / alpha_0)
+        // g(n) / g(n_0): SIN alpha / alpha_0, ZEA exp(i Im la), TAN (alpha /
+        // alpha_0) / (1 + x), x = 2 (n - n_0) / (2 n_0 - 1), n = n_0 exp(2 Re la).
+        const cf z1 = la.l1;
+        const cf z2 = cf{A2[0], A2[3]} * inv_a, z3 = cf{A3[0], A3[3]} * inv_a;
+        cf e1, e2, e3;
+        float g = 2.f, h = 1.1f * ta.X;   // h: size of e - 1 at the chunk's end
+        rx = 2.2f;
+        if (coord == SO3G_COORD_TAN) {
+            const float ct = 2.f * al2 - 1.f;
+            if (!(ct > 0.1f)) return;
+            const float ic = rcp_approx(ct), f = 2.f * al2 * ic;
+            const float p1 = 2.f * la.l1.r, p2 = 2.f * la.l2.r, p3 = 2.f * la.l3.r;
+            const float x1 = f * p1, x2 = f * (p2 + 0.5f * p1 * p1),
+                        x3 = f * (p3 + p1 * p2 + (1.f / 6.f) * p1 * p1 * p1);
+            const float g1 = -x1, g2 = x1 * x1 - x2, g3 = 2.f * x1 * x2 - x3 - x1 * x1 * x1;
+            e1 = z1 + cf{g1, 0.f};
+            e2 = z2 + g1 * z1 + cf{g2, 0.f};
+            e3 = z3 + g1 * z2 + g2 * z1 + cf{g3, 0.f};
+            g *= ic;
+            h += 2.4f * f * ta.X;
+            rx = 2.4f * ic * ic;
+        } else if (coord == SO3G_COORD_ZEA) {
+            const float t1 = la.l1.i, t2 = la.l2.i, t3 = la.l3.i;
+            e1 = cf{0.f, t1};
+            e2 = cf{-0.5f * t1 * t1, t2};
+            e3 = cf{-t1 * t2, t3 - (1.f / 6.f) * t1 * t1 * t1};
+            g *= rsqrtf(al2);
+            rx = 2.4f * ia;
+        } else {
+            e1 = z1;
+            e2 = z2;
+            e3 = z3;
+        }
+        if (!(h < 0.1f)) return;
+        ry = rx;
+        const cf b0{A[2], -A[1]}, b1{A1[2], -A1[1]}, b2{A2[2], -A2[1]}, b3{A3[2], -A3[1]};
+        const cf s = g * cf{A[0], A[3]};
+        const cf p1 = s * (b1 + e1 * b0), p2 = s * (b2 + e1 * b1 + e2 * b0),
+                 p3 = s * (b3 + e1 * b2 + e2 * b1 + e3 * b0);
+        cy1 = p1.r;
+        cy2 = p2.r;
+        cy3 = p3.r;
+        cx1 = -p1.i;
+        cx2 = -p2.i;
+        cx3 = -p3.i;
+        // Order >= 4 of e times beta: with bk = |b_k| / 2^k and e's terms of
+        // order n below 2 h^n (h covers alpha's, the exponential's and TAN's
+        // series at the chunk's end).
+        const float k0 = cf_abs(b0), k1 = 0.5f * cf_abs(b1), k2 = 0.25f * cf_abs(b2),
+                    k3 = 0.125f * cf_abs(b3), k4 = 0.0625f * cf_abs(cf{A4[2], A4[1]});
+        const float h2 = h * h;
+        tx = ty = g * (4.f * (k0 * h2 * h2 + k1 * h2 * h + k2 * h2 + k3 * h) + 1.2f * k4) *
+                      1.2f + 1e-12f;
+    }
+    // Pixel coordinates: the coefficients' float32 errors (24u of the terms'
+    // sizes, of which cx1 .. carry products of at most a few factors), the
+    // sample's polynomial (6u of its terms).
+    const float icx = HP ? 1.f : a.mc.inv_cdx, icy = HP ? 1.f : a.mc.inv_cdy;
+    const float aix = fabsf(icx), aiy = fabsf(icy);
+    const float sx = 0.5f * fabsf(cx1) + 0.25f * fabsf(cx2) + 0.125f * fabsf(cx3);
+    const float sy = 0.5f * fabsf(cy1) + 0.25f * fabsf(cy2) + 0.125f * fabsf(cy3);
+    const float big = CL == CX_CAR ? ta.X * 4.f + sx + sy + zz
+                                   : 4.f * (ta.X + 0.5f * cf_abs(cf{A1[2], A1[1]})) * (1.f + rx);
+    float ex = (tx + lutx + rx * E + 32.f * u * (sx + big)) * aix;
+    float ey = (ty + luty + ry * E + 32.f * u * (sy + big)) * aiy;
+    int xb = 0, yb = 0;
+    float xf, yf;
+    if constexpr (HP) {
+        xf = X0.hi + X0.lo;
+        yf = Y0.hi + Y0.lo;
+        ex = 1.5f * (ex + 3.f * u * (fabsf(xf) + sx) + 1e-11f);
+        ey = 1.5f * (ey + 3.f * u * (fabsf(yf) + sy) + 1e-11f);
+    } else {
+        const dfl xa = df_add(df_mul(X0, a.fc.inv_cdx), a.fc.off_x);
+        const dfl ya = df_add(df_mul(Y0, a.fc.inv_cdy), a.fc.off_y);
+        if (!(fabsf(xa.hi) < 1e7f && fabsf(ya.hi) < 1e7f && sx * aix < 1e5f && sy * aiy < 1e5f))
+            return;
+        dfl fx, fy;
+        xb = df_floor(xa, fx);
+        yb = df_floor(ya, fy);
+        xf = (fx.hi - 0.5f) + fx.lo;
+        yf = (fy.hi - 0.5f) + fy.lo;
+        xb -= kCxMagicBits;
+        yb -= kCxMagicBits;
+        // 2 kEpsPix: the reference's own rounding and the middle's error; u:
+        // the final sum's rounding.
+        ex = 1.5f * (ex + 2.f * kEpsPix + 2.f * u);
+        ey = 1.5f * (ey + 2.f * kEpsPix + 2.f * u);
+    }
+    constexpr float s1 = 1.f / 64.f, s2 = s1 * s1, s3 = s2 * s1, s4 = s2 * s2;
+    w[0] = make_float4(xf, cx1 * icx * s1, cx2 * icx * s2, cx3 * icx * s3);
+    w[1] = make_float4(yf, cy1 * icy * s1, cy2 * icy * s2, cy3 * icy * s3);
+    float e = 0.f;
+    bool flag = false;
+    if constexpr (SPIN) {
+        // The spin factors at the middle, F1 + i F2 = P v^2 / D, and phi's
+        // derivative there, 2 (Im(alpha_1 conj(alpha_0)) / |alpha_0|^2 + ...
+        // beta) or 4 Im(alpha_1 conj(alpha_0)) / |alpha_0|^2, double-float.
+        const dfl invD = df_recip(D);
+        const dfl F1 = df_mulf(df_mul(df_dot<2>({Nc, Ns}, {Nc, df_neg(Ns)}), invD), Pr);
+        const dfl F2 = df_mulf(df_mul(df_mulf(df_mul(Nc, Ns), 2.f), invD), Pr);
+        dfl ph;
+        {
+            const float4 h = __ldg(&cb.a1_hi), l = __ldg(&cb.a1_lo);
+            const dfl q[4] = {{h.x, l.x}, {h.y, l.y}, {h.z, l.z}, {h.w, l.w}};
+            dfl p, r, s, t;
+            df_qmul(q, qd, p, r, s, t);
+            const dfl na = df_dot<2>({qa, qe}, {qa, qe});
+            ph = df_mul(df_dot<2>({t, p}, {qa, df_neg(qe)}), df_recip(na));
+            if (CL == CX_CAR) {
+                const dfl nb = df_dot<2>({qb, qc}, {qb, qc});
+                ph = df_add(ph, df_mul(df_dot<2>({r, s}, {qc, df_neg(qb)}), df_recip(nb)));
+                ph = df_mulf(ph, 2.f);
+            } else {
+                ph = df_mulf(ph, 4.f);
+            }
+        }
+        // exp(i (phi1 u + phi2 u^2 + ...)) - 1 = sum of (cr_k + i ci_k) u^k;
+        // its first coefficient i phi1, the second -phi1^2 / 2 + i phi2.
+        const dfl hp2 = df_mulf(df_mul(ph, ph), -0.5f);
+        const float p1 = ph.hi, pp = p1 * p1;
+        const cf c3{-p1 * phi2, phi3 - (1.f / 6.f) * pp * p1};
+        const cf c4{-p1 * phi3 - 0.5f * phi2 * phi2 + (1.f / 24.f) * pp * pp,
+                    phi4 - 0.5f * pp * phi2};
+        // f0, f1 rounded to multiples of gr = 2^-22 of the power of two
+        // >= |Pr|, so that f0 + k f1 (|k| <= 32, |sum| below twice that power)
+        // is exact; the rest, l0 and l1, and the higher terms go into the
+        // float32 correction.
+        const float aP = fabsf(Pr);
+        const int pe = ((__float_as_int(aP) - 1) >> 23) + 1;   // biased exponent
+        const bool fine = pe > 24 && pe < 250 && fabsf(p1) < 0.5f;
+        const float cst = fine ? 3.f * __int_as_float(pe << 23) : 0.f;
+        const float gr = fine ? __int_as_float((pe - 22) << 23) : 0.f;
+#pragma unroll
+        for (int f = 0; f < 2; f++) {
+            // F1's terms: Re(c_k (F1 + i F2)); F2's: Im.
+            const dfl F = f == 0 ? F1 : F2, G = f == 0 ? df_neg(F2) : F1;
+            const dfl d1 = df_mul(ph, G);
+            const dfl q1{d1.hi * s1, d1.lo * s1};
+            const float f0 = (F.hi + cst) - cst, f1 = (q1.hi + cst) - cst;
+            const float l0 = (F.hi - f0) + F.lo, l1 = (q1.hi - f1) + q1.lo;
+            const float a2 = fmaf(phi2, G.hi, df_mul(hp2, F).hi);
+            const float a3 = c3.r * F.hi + c3.i * G.hi, a4 = c4.r * F.hi + c4.i * G.hi;
+            w[4 + 2 * f] = make_float4(f0, f1, l0, l1);
+            w[5 + 2 * f] = make_float4(a2 * s2, a3 * s3, a4 * s4, 0.f);
+        }
+        // e: the double-float error and the reference's roundings (kEpsPf;
+        // phi1's is of the same size), the terms left out, a norm off 1
+        // (CAR's reference divides by (1 - sin^2) / 4, the model by
+        // |alpha beta|^2), the float32 errors of phi2 (16u |z1|^2), phi3,
+        // phi4 and of the products, the correction's roundings (3u of its
+        // terms), and the boresight's distance from Q.
+        const float h1 = 0.5f * fabsf(p1), h2 = 0.25f * fabsf(phi2) + u * zz,
+                    h3 = 0.125f * fabsf(phi3) + 8.f * u * zz, h4 = 0.0625f * fabsf(phi4) + 8.f * u * zz;
+        const CxTail tp = cx_tail(h1, h2, h3, h4);
+        const float Df = D.hi;
+        const dfl qq = df_dot<4>(qd, qd);
+        const float eta = __ldg(&cb.eta) + fabsf((qq.hi - 1.f) + qq.lo);
+        e = 1.2f * (cx_tail_exp(tp) + 4.f * tail) +
+            kEpsPf * fmaxf(1.f, 0.25f / Df) * (1.f + h1) + (CL == CX_CAR ? 0.6f * eta / Df : 0.f) +
+            u * (3.f * h1 * h1 + 8.f * h2 + 4.f * zz + 16.f * (h3 + h4 + h1 * (h2 + h1 * h1)));
+        e = e * fmaxf(aP, 1e-3f) + 3.f * u * 18.f * gr;
+        if (lsb > 0.f) {
+            // The residual's turn: gradient at both ends, linear between;
+            // second order in the residual; its quantisation; float32.
+            flag = true;
+            float N0[4], N1[4], g0[3], g1[3];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                N0[c] = A[c] - 0.5f * A1[c] + 0.25f * A2[c];
+                N1[c] = A[c] + 0.5f * A1[c] + 0.25f * A2[c];
+            }
+            const float ka = cx_gradient<CL>(N0, d32, g0), kb = cx_gradient<CL>(N1, d32, g1);
+            const float km = fmaxf(ka, kb) + 1.f;
+            e += aP * (E * (2.1f * gerr + km * (64.f * u + 4.f * eta)) + 16.f * km * km * E * E +
+                       2.f * (km + 4.f) * lsb);
+            const float hm = 0.5f * lsb, hd = lsb * s1;
+            w[5].w = (g0[0] + g1[0]) * hm;
+            w[7].w = (g0[1] + g1[1]) * hm;
+            w[8] = make_float4((g0[2] + g1[2]) * hm, (g1[0] - g0[0]) * hd, (g1[1] - g0[1]) * hd,
+                               (g1[2] - g0[2]) * hd);
+        } else {
+            e += aP * (4.3f + 2.2f * rsqrtf(Df)) * E;
+        }
+        if (!fine) e = __int_as_float(0x7f800000);   // never certain
+    }
+    w[2] = make_float4(HP ? ex : 0.5f - ex, HP ? ey : 0.5f - ey, e, 0.f);
+    w[3] = make_float4(__int_as_float(xb), __int_as_float(yb), __int_as_float(mid),
+                       flag ? 1.f : 0.f);
+}
+
+// The exact part and the correction of a spin factor at k = t - mid.
+__device__ __forceinline__ void cx_factor(const float4 &A, const float4 &B, float k, float &S,
+                                          float &L) {
+    L = fmaf(k, fmaf(k, fmaf(k, fmaf(k, B.z, B.y), B.x), A.w), A.z);
+    S = fmaf(k, A.y, A.x);
+}
+
+// One sample (k = t - mid) of a modelled chunk: pixel key (flat: iy * nx +
+// ix, of the parent map when tiled; HEALPix: the pixel), on the map or not,
+// and the spin factors of an NC-component map; false when the pixel or
+// (on the map) a spin factor is not certain.  res: the sample's residual
+// (used where the chunk's flag is set).  P = PX_FLAT_T_NN: the tiled
+// pixelizor's rule (int() truncation, src/Projection.cxx:1124-1138).
+// A spin factor is within e of S + L (S exact), so the reference's value
+// rounds to the same float32 when S + (L + e) and S + (L - e) do.
+template <int P, int NC>
+__device__ __forceinline__ bool cx_sample(const float4 *w, float k, const float (&res)[3],
+                                          bool flag, const DGeom &g, float T, int &key, bool &on,
+                                          float (&pf)[3]) {
+    const float4 P0 = w[0], P1 = w[1], P2 = w[2];
+    const float x = fmaf(k, fmaf(k, fmaf(k, P0.w, P0.z), P0.y), P0.x);
+    const float y = fmaf(k, fmaf(k, fmaf(k, P1.w, P1.z), P1.y), P1.x);
+    bool ok;
+    if constexpr (P == PX_HP_NT || P == PX_HP_T) {
+        int pix[1] = {0};
+        ok = P2.x >= 0.f && hp_pixel_f32<P, P == PX_HP_T, true>(g, x, P2.x, y, P2.y, 0.f, 0.f, pix);
+        key = pix[0];
+        on = true;
+    } else {
+        const float4 P3 = w[3];
+        // x, y less 1/2: the nearest integer is the floor, and the distance
+        // from it the fraction less 1/2.
+        const float rx = x + kCxMagic, ry = y + kCxMagic;
+        ok = (fabsf(x - (rx - kCxMagic)) < P2.x) & (fabsf(y - (ry - kCxMagic)) < P2.y);
+        int ix = __float_as_int(P3.x) + __float_as_int(rx),
+            iy = __float_as_int(P3.y) + __float_as_int(ry);
+        if constexpr (P == PX_FLAT_T_NN) {
+            on = ((unsigned)(ix + 1) < (unsigned)(g.nx + 1)) &
+                 ((unsigned)(iy + 1) < (unsigned)(g.ny + 1));
+            ix = max(ix, 0);
+            iy = max(iy, 0);
+        } else {
+            on = ((unsigned)ix < (unsigned)g.nx) & ((unsigned)iy < (unsigned)g.ny);
+        }
+        key = iy * g.nx + ix;
+    }
+    if constexpr (NC == 1) {
+        pf[0] = T;
+        pf[1] = pf[2] = 0.f;
+    } else {
+        float S1, L1, S2, L2;
+        const float4 W5 = w[5], W7 = w[7];
+        cx_factor(w[4], W5, k, S1, L1);
+        cx_factor(w[6], W7, k, S2, L2);
+        if (flag) {
+            const float4 W8 = w[8];
+            const float dphi = fmaf(fmaf(k, W8.y, W5.w), res[0],
+                                    fmaf(fmaf(k, W8.z, W7.w), res[1], fmaf(k, W8.w, W8.x) * res[2]));
+            L1 = fmaf(-S2, dphi, L1);
+            L2 = fmaf(S1, dphi, L2);
+        }
+        const float v1 = S1 + (L1 + P2.z), v2 = S2 + (L2 + P2.z);
+        const bool c = (v1 == S1 + (L1 - P2.z)) & (v2 == S2 + (L2 - P2.z));
+        ok = ok & (c | !on);
+        if constexpr (NC == 2) {
+            pf[0] = v1;
+            pf[1] = v2;
+            pf[2] = 0.f;
+        } else {
+            pf[0] = T;
+            pf[1] = v1;
+            pf[2] = v2;
+        }
+    }
+    return ok;
+}
+
+// The residuals of samples t .. t + 3 (t a multiple of 4).
+__device__ __forceinline__ void cx_residuals(const short4 *resid, int t, float (&r)[4][3]) {
+    const int4 *p = reinterpret_cast<const int4 *>(resid + t);
+    const int4 u = __ldg(p), v = __ldg(p + 1);
+    const int lo[4] = {u.x, u.z, v.x, v.z}, hi[4] = {u.y, u.w, v.y, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        r[i][0] = (float)(short)(lo[i] & 0xffff);
+        r[i][1] = (float)(lo[i] >> 16);
+        r[i][2] = (float)(short)(hi[i] & 0xffff);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Samples the models leave.  Each warp collects them in shared memory and
+// appends them, 32 or more at a time, to a list in global memory; a second
+// kernel takes the list through the per-sample certified path and appends
+// what that leaves to another list, for the float64 path: every path runs
+// on full warps, and the main kernel's code stays small (with the per-sample
+// paths called from it, instruction fetch stalls made it 2.2 times slower).
+// Entries past a list's capacity are handled on the spot.
+
+struct CxList {
+    unsigned long long *count;
+    int2 *entry;               // (det, t)
+    unsigned long long cap;
+};
+
+// Samples a warp collects before it appends them: below 32 plus a round.
+constexpr int kCxQueue = 160;
+
+struct CxWarp {
+    int n;                   // entries of queue
+    int queue[kCxQueue];
+};
+
+// Appends samples tq + i for the bits i of f4; all lanes must call when any
+// has a bit.  Returns the queue's length.
+__device__ __forceinline__ int cx_enqueue(CxWarp &cw, unsigned f4, int tq) {
+    if (f4) {
+        int p = atomicAdd(&cw.n, __popc(f4));
+        while (f4) {
+            cw.queue[p++] = tq + __ffs(f4) - 1;
+            f4 &= f4 - 1;
+        }
+    }
+    __syncwarp();
+    return cw.n;
+}
+
+// Moves the warp's queue to the list; over(t) handles a sample that does
+// not fit.  All lanes must call.
+template <class F>
+__device__ __forceinline__ void cx_append(CxWarp &cw, const CxList &list, int det, F &&over) {
+    const int lane = threadIdx.x & 31, n = cw.n;
+    if (n == 0) return;
+    unsigned long long p = 0;
+    if (lane == 0) p = atomicAdd(list.count, (unsigned long long)n);
+    p = __shfl_sync(kFull, p, 0);
+    for (int i = lane; i < n; i += 32) {
+        if (p + i < list.cap) list.entry[p + i] = make_int2(det, cw.queue[i]);
+        else over(cw.queue[i]);
+    }
+    __syncwarp();
+    if (lane == 0) cw.n = 0;
+    __syncwarp();
+}
+
+// Calls f(det, t) for every entry of `list`, one lane each; where f returns
+// false, the entry goes to `next` (over(det, t) when that is full).
+template <class F, class G>
+__device__ __forceinline__ void cx_for_each(const CxList &list, const CxList &next, F &&f,
+                                            G &&over) {
+    const unsigned long long n = min(*list.count, list.cap);
+    const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
+    const int lane = threadIdx.x & 31;
+    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+         (i & ~31ULL) < n; i += stride) {
+        int2 e = make_int2(0, 0);
+        bool left = false;
+        if (i < n) {
+            e = list.entry[i];
+            left = !f(e.x, e.y);
+        }
+        const unsigned m = __ballot_sync(kFull, left);
+        if (!m) continue;
+        unsigned long long p = 0;
+        if (lane == 0) p = atomicAdd(next.count, (unsigned long long)__popc(m));
+        p = __shfl_sync(kFull, p, 0) + __popc(m & ((1u << lane) - 1u));
+        if (left) {
+            if (p < next.cap) next.entry[p] = e;
+            else over(e.x, e.y);
+        }
+    }
+}
+
+constexpr unsigned kCxFixBlocks = 152 * 8;   // of kBlock threads, striding over a list
+
+// Samples per block of a call: each warp of a block takes up to kCxGroup
+// chunks at once, fewer (even) when the call would not fill the GPU twice.
+inline int cx_piece(long long n_seg, long long max_len) {
+    constexpr int kWarps = kBlock / 32;
+    const long long chunks = n_seg * ((max_len + kCxLen - 1) / kCxLen);
+    long long per_warp = chunks / (2LL * 152 * 4 * kWarps);
+    per_warp = per_warp < 2 ? 2 : (per_warp > kCxGroup ? kCxGroup : per_warp & ~1LL);
+    long long p = per_warp * kWarps * kCxLen;
+    if (per_warp == kCxGroup && chunks > 16LL * 152 * 4 * kWarps * kCxGroup) p *= 2;
+    while ((max_len + p - 1) / p > 65535) p *= 2;
+    return (int)p;
+}
+
+// The workspace of a call, in stream-ordered memory: the chunks' boresight
+// models, the residuals and the two lists (one entry for every 24 and 96
+// samples: the workloads leave 1 in 50 and 1 in 1000).
+struct CxWork {
+    void *mem = nullptr;
+    CxModel model;
+    CxList left, exact;
+    SkipIf gate;               // the chunked kernels skip when it holds
+};
+
+// Allocates the workspace and makes the boresight models; false (nothing
+// left allocated) when that fails (the caller takes the per-sample path).
+inline bool cx_work(CxWork &w, const double *bore, int n_time, long long samples,
+                    cudaStream_t stream) {
+    const long long n_chunks = (n_time + kCxLen - 1) / kCxLen;
+    const long long cap1 = samples / 24 + 4096, cap2 = samples / 96 + 4096;
+    const size_t o_res = 256 + sizeof(CxBore) * (size_t)n_chunks;
+    const size_t o_l1 = o_res + sizeof(short4) * (size_t)(n_chunks * kCxLen);
+    const size_t o_l2 = o_l1 + sizeof(int2) * (size_t)cap1;
+    const size_t bytes = o_l2 + sizeof(int2) * (size_t)cap2;
+    if (cudaMallocAsync(&w.mem, bytes, stream) != cudaSuccess) {
+        cudaGetLastError();
+        w.mem = nullptr;
+        return false;
+    }
+    char *p = static_cast<char *>(w.mem);
+    unsigned long long *counts = reinterpret_cast<unsigned long long *>(p);
+    CxBore *models = reinterpret_cast<CxBore *>(p + 256);
+    short4 *resid = reinterpret_cast<short4 *>(p + o_res);
+    w.model = CxModel{models, resid};
+    w.left = CxList{counts, reinterpret_cast<int2 *>(p + o_l1), (unsigned long long)cap1};
+    w.exact = CxList{counts + 1, reinterpret_cast<int2 *>(p + o_l2), (unsigned long long)cap2};
+    unsigned *rough = reinterpret_cast<unsigned *>(counts + 2);
+    w.gate = SkipIf{rough, (unsigned)(n_chunks / 4), true};
+    bool ok = cudaMemsetAsync(counts, 0, 256, stream) == cudaSuccess;
+    if (ok) {
+        const long long threads = 16 * n_chunks;
+        k_cx_bore<<<(unsigned)((threads + 127) / 128), 128, 0, stream>>>(bore, n_time,
+                                                                        (int)n_chunks, models, resid,
+                                                                        rough);
+        ok = after_launch("boresight chunk models (certified)") == SO3G_OK;
+    }
+    if (!ok) {
+        cudaGetLastError();
+        cudaFreeAsync(w.mem, stream);
+        w.mem = nullptr;
+        clear_error();
+    }
+    return ok;
+}
+
+}  // namespace
+
+}  // namespace so3g

@@ -578,8 +578,7 @@ __device__ __forceinline__ double f2d(float f) {
     const unsigned u = __float_as_uint(f);
     const unsigned a = u & 0x7fffffffu;
     if (a - 0x00800000u < 0x7f000000u)
-        return __hiloint2double((int)((u & 0x80000000u) | ((a >> 3) + (896u << 20))),
-                                (int)(u << 29));
+        return __hiloint2double((((int)u >> 3) & (int)0x8fffffffu) + (896 << 20), (int)(u << 29));
     if (a == 0u) return __hiloint2double((int)(u & 0x80000000u), 0);
     return f2d_special(f);
 }
@@ -642,6 +641,17 @@ __device__ __forceinline__ void flush_runs(long long key, long long plane, float
             if ((vmask >> k) & 1u) atomicAdd(map + key + mult[k] * plane, f2d(v[k]) + f2d(e[k]));
     }
 }
+
+// A kernel's device-side gate: it returns at once when *count > limit (skip)
+// or when *count <= limit (!skip); none when count is NULL.
+struct SkipIf {
+    const unsigned *count = nullptr;
+    unsigned limit = 0;
+    bool skip = false;
+    __device__ __forceinline__ bool holds() const {
+        return count && (__ldg(count) > limit) == skip;
+    }
+};
 
 // Sample-range work decomposition shared by the projection kernels: block
 // (x, y) covers piece y of segment x, `piece` samples long.

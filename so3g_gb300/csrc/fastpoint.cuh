@@ -52,7 +52,12 @@ __device__ __forceinline__ int warp_enqueue(int *q, int qn, bool push, int t) {
 
 // Bounds of |double-float value - reference float64 value|.
 constexpr float kEpsPix = 1e-7f;        // pixel coordinate units
-constexpr float kEpsPf = 1e-11f;        // spin factors (values of order 1)
+// Spin factors (of order 1).  df_split keeps 2^-46 of each input, so the
+// quaternion product's components are within 6e-14, alpha = a + id and beta
+// = c + ib within 8e-14, v = alpha beta (Nc + i Ns) within 1.2e-13 and sin(lat)
+// within 2.3e-13; P v^2 / D is then within 1.1e-12 max(1, 1/(4D)) P, the
+// zenithal P (alpha^2 / n)^2 within 5e-13 / sqrt(n).
+constexpr float kEpsPf = 3e-12f;
 
 struct dfl {
     float hi, lo;
@@ -263,6 +268,93 @@ __device__ __forceinline__ bool fast_lon_spin(const FastTables &ft, const FastCo
     return true;
 }
 
+// Zenithal quantities of q = (a, b, c, d): n = a^2 + d^2 = cos^2(theta/2),
+// u = a*b - c*d, v = a*c + b*d.
+__device__ __forceinline__ void fast_zen_nuv(const dfl &a, const dfl &b, const dfl &c,
+                                             const dfl &d, dfl &n, dfl &u, dfl &v) {
+    n = df_dot<2>({a, d}, {a, d});
+    u = df_dot<2>({a, c}, {b, df_neg(d)});
+    v = df_dot<2>({a, b}, {c, d});
+}
+
+// Their spin quantities: coords[2] = (a^2 - d^2)/n, coords[3] = 2ad/n.
+__device__ __forceinline__ void fast_zen_spin(const dfl &a, const dfl &d, const dfl &n, dfl &Nc,
+                                              dfl &Ns, dfl &D) {
+    Nc = df_dot<2>({a, d}, {a, df_neg(d)});
+    Ns = df_mulf(df_mul(a, d), 2.f);
+    D = df_mul(n, n);
+}
+
+// Projection-plane coordinates of the zenithal projections; false far from
+// the pole (see fast_native).
+template <int C>
+__device__ __forceinline__ bool fast_zen_xy(const FastTables &ft, const FastConst &fc,
+                                            const dfl &b, const dfl &c, const dfl &n,
+                                            const dfl &u, const dfl &v, dfl &X, dfl &Y) {
+    if (C == SO3G_COORD_TAN) {
+        // :372-400: X = 2u / cos(theta), cos(theta) = 2n - 1.
+        const dfl ct = df_sub(df_mulf(n, 2.f), dfl{1.f, 0.f});
+        if (!(ct.hi > 1e-2f)) return false;
+        const dfl r = df_mulf(df_recip(ct), 2.f);
+        X = df_mul(u, r);
+        Y = df_mul(v, r);
+    } else if (C == SO3G_COORD_ZEA) {
+        // :408-437: X = 2u / sqrt(n).
+        if (!(n.hi > 1e-4f)) return false;
+        const float s0 = sqrtf(n.hi);
+        const float res = fmaf(-s0, s0, n.hi) + n.lo;   // n - s0^2
+        const dfl sq = fast_two_sum(s0, res / (2.f * s0));
+        const dfl r = df_mulf(df_recip(sq), 2.f);
+        X = df_mul(u, r);
+        Y = df_mul(v, r);
+    } else if (C == SO3G_COORD_ARC) {
+        // :284-326: h = sqrt(sc^2 + ss^2) (sc = a*c + b*d, ss = a*b -
+        // c*d), R = ASIN(2 h) / h, or pi / h - R where a^2 + d^2 <
+        // b^2 + c^2; X = ss R, Y = sc R.  The exact path takes the
+        // reference's series branch (h < 1e-8) and the neighbourhoods
+        // of its two decisions: h < 1e-6, |(a^2 + d^2) - (b^2 + c^2)| <=
+        // 1e-6, and 2 h near 1 (the table's end, theta near 90 deg).
+        if (!(n.hi > 1e-4f)) return false;
+        const dfl h2 = df_dot<2>({u, v}, {u, v});
+        if (!(h2.hi > 1e-12f)) return false;
+        const dfl s2 = df_dot<2>({b, c}, {b, c});
+        const dfl dcs = df_sub(n, s2);
+        if (!(fabsf(dcs.hi) > 1e-6f)) return false;
+        const float h0 = sqrtf(h2.hi);
+        const dfl h = fast_two_sum(h0, (fmaf(-h0, h0, h2.hi) + h2.lo) / (2.f * h0));
+        const dfl x2 = df_mulf(h, 2.f);
+        if (!(x2.hi < 0.998f)) return false;
+        const dfl ih = df_recip(h);
+        dfl R = df_mul(lut_df(ft.asin_t, x2), ih);
+        if (dcs.hi < 0.f) R = df_sub(df_mul(fc.pi, ih), R);
+        X = df_mul(u, R);
+        Y = df_mul(v, R);
+    } else {
+        // SIN, :337-364: X = 2u, Y = 2v.
+        if (!(n.hi > 1e-4f)) return false;
+        X = df_mulf(u, 2.f);
+        Y = df_mulf(v, 2.f);
+    }
+    return true;
+}
+
+// CAR coordinates and spin quantities of q = (a, b, c, d).
+__device__ __forceinline__ bool fast_car(const FastTables &ft, const FastConst &fc, const dfl &a,
+                                         const dfl &b, const dfl &c, const dfl &d, dfl &X, dfl &Y,
+                                         dfl &Nc, dfl &Ns, dfl &D) {
+    // cos(theta) = a^2 - b^2 - c^2 + d^2 = sin(lat).
+    const dfl cos_t = df_dot<4>({a, b, c, d}, {a, df_neg(b), df_neg(c), d});
+    // Near the native poles (|lat| > ~87 deg) the tables' ends and the
+    // spin factors are ill-conditioned: exact path.
+    if (!(fabsf(cos_t.hi) < 0.998f)) return false;
+    // lat = ASIN(cos_t) (odd, continuous at 0).
+    const bool south = cos_t.hi < 0.f;
+    dfl lat = lut_df(ft.asin_t, south ? df_neg(cos_t) : cos_t);
+    if (south) lat = df_neg(lat);
+    Y = lat;
+    return fast_lon_spin(ft, fc, a, b, c, d, cos_t, X, Nc, Ns, D);
+}
+
 template <int C>
 __device__ __forceinline__ bool fast_native(const FastTables &ft, const FastConst &fc,
                                             const dfl (&qb)[4], const dfl (&qd)[4], dfl &X,
@@ -270,70 +362,12 @@ __device__ __forceinline__ bool fast_native(const FastTables &ft, const FastCons
     dfl a, b, c, d;
     df_qmul(qb, qd, a, b, c, d);
     if (C == SO3G_COORD_CAR) {
-        // cos(theta) = a^2 - b^2 - c^2 + d^2 = sin(lat).
-        const dfl cos_t = df_dot<4>({a, b, c, d}, {a, df_neg(b), df_neg(c), d});
-        // Near the native poles (|lat| > ~87 deg) the tables' ends and the
-        // spin factors are ill-conditioned: exact path.
-        if (!(fabsf(cos_t.hi) < 0.998f)) return false;
-        // lat = ASIN(cos_t) (odd, continuous at 0).
-        const bool south = cos_t.hi < 0.f;
-        dfl lat = lut_df(ft.asin_t, south ? df_neg(cos_t) : cos_t);
-        if (south) lat = df_neg(lat);
-        Y = lat;
-        return fast_lon_spin(ft, fc, a, b, c, d, cos_t, X, Nc, Ns, D);
+        return fast_car(ft, fc, a, b, c, d, X, Y, Nc, Ns, D);
     } else {
-        // Zenithal: cos^2(theta/2) = a^2 + d^2; coords[2] = (a^2 - d^2)/n,
-        // coords[3] = 2ad/n.
-        const dfl n = df_dot<2>({a, d}, {a, d});
-        const dfl u = df_dot<2>({a, c}, {b, df_neg(d)});   // a*b - c*d
-        const dfl v = df_dot<2>({a, b}, {c, d});           // a*c + b*d
-        if (C == SO3G_COORD_TAN) {
-            // :372-400: X = 2u / cos(theta), cos(theta) = 2n - 1.
-            const dfl ct = df_sub(df_mulf(n, 2.f), dfl{1.f, 0.f});
-            if (!(ct.hi > 1e-2f)) return false;
-            const dfl r = df_mulf(df_recip(ct), 2.f);
-            X = df_mul(u, r);
-            Y = df_mul(v, r);
-        } else if (C == SO3G_COORD_ZEA) {
-            // :408-437: X = 2u / sqrt(n).
-            if (!(n.hi > 1e-4f)) return false;
-            const float s0 = sqrtf(n.hi);
-            const float res = fmaf(-s0, s0, n.hi) + n.lo;   // n - s0^2
-            const dfl sq = fast_two_sum(s0, res / (2.f * s0));
-            const dfl r = df_mulf(df_recip(sq), 2.f);
-            X = df_mul(u, r);
-            Y = df_mul(v, r);
-        } else if (C == SO3G_COORD_ARC) {
-            // :284-326: h = sqrt(sc^2 + ss^2) (sc = a*c + b*d, ss = a*b -
-            // c*d), R = ASIN(2 h) / h, or pi / h - R where a^2 + d^2 <
-            // b^2 + c^2; X = ss R, Y = sc R.  The exact path takes the
-            // reference's series branch (h < 1e-8) and the neighbourhoods
-            // of its two decisions: h < 1e-6, |(a^2 + d^2) - (b^2 + c^2)| <=
-            // 1e-6, and 2 h near 1 (the table's end, theta near 90 deg).
-            if (!(n.hi > 1e-4f)) return false;
-            const dfl h2 = df_dot<2>({u, v}, {u, v});
-            if (!(h2.hi > 1e-12f)) return false;
-            const dfl s2 = df_dot<2>({b, c}, {b, c});
-            const dfl dcs = df_sub(n, s2);
-            if (!(fabsf(dcs.hi) > 1e-6f)) return false;
-            const float h0 = sqrtf(h2.hi);
-            const dfl h = fast_two_sum(h0, (fmaf(-h0, h0, h2.hi) + h2.lo) / (2.f * h0));
-            const dfl x2 = df_mulf(h, 2.f);
-            if (!(x2.hi < 0.998f)) return false;
-            const dfl ih = df_recip(h);
-            dfl R = df_mul(lut_df(ft.asin_t, x2), ih);
-            if (dcs.hi < 0.f) R = df_sub(df_mul(fc.pi, ih), R);
-            X = df_mul(u, R);
-            Y = df_mul(v, R);
-        } else {
-            // SIN, :337-364: X = 2u, Y = 2v.
-            if (!(n.hi > 1e-4f)) return false;
-            X = df_mulf(u, 2.f);
-            Y = df_mulf(v, 2.f);
-        }
-        Nc = df_dot<2>({a, d}, {a, df_neg(d)});
-        Ns = df_mulf(df_mul(a, d), 2.f);
-        D = df_mul(n, n);
+        dfl n, u, v;
+        fast_zen_nuv(a, b, c, d, n, u, v);
+        if (!fast_zen_xy<C>(ft, fc, b, c, n, u, v, X, Y)) return false;
+        fast_zen_spin(a, d, n, Nc, Ns, D);
         return true;
     }
 }

@@ -13,32 +13,13 @@
 // exact path's.
 
 #include "host.h"
+#include "gather_kernel.cuh"
 #include "interp_point.cuh"
 #include "mx_common.cuh"
 
 namespace so3g {
 
 namespace {
-
-
-struct GatherArgs {
-    DGeom g;
-    const double *bore;
-    const double *dets;
-    const float *resp;
-    const double *map;
-    float *signal;
-    long long sig_stride;
-    Segs segs;
-    int piece;
-    int *err;
-    int fast;           // SO3G_POINTING_*: 0 exact, 1 certified, 2 mixed
-    FastTables ft;
-    FastConst fc;
-    MixedConst mc;
-    const float4 *bore32;   // float32 boresight (mixed pointing), or NULL
-    const float4 *map32;    // float32 (T, Q, U, 0) per pixel (mixed pointing), or NULL
-};
 
 // Largest parent map (pixels) that gets the float32 copy when tiled: the
 // copy spans the parent map (16 bytes per pixel), present tiles or not.
@@ -101,43 +82,6 @@ __global__ void k_map_f32(const double *map, int nc, long long npix, float4 *out
     out[i] = make_float4(v[0], v[1], v[2], 0.f);
 }
 
-// Adds the sample's map terms to its signal (src/Projection.cxx:1763-1765).
-template <int P, int NT>
-__device__ __forceinline__ void gather_taps(const GatherArgs &a, float *sp, int n,
-                                            const int (*pix)[3], const float *w,
-                                            const float *pf) {
-    float sig = *sp;
-    const int nc = a.g.ncomp;
-#pragma unroll
-    for (int k = 0; k < NT; k++) {
-        if (k >= n) break;
-        long long off, plane;
-        int bad = locate<P>(a.g, pix[k], &off, &plane);
-        if (bad >= 0) {
-            record_missing_tile(a.err, bad);
-            continue;
-        }
-#pragma unroll
-        for (int c = 0; c < 3; c++)
-            if (c < nc) sig += __ldg(a.map + off + c * plane) * pf[c] * w[k];
-    }
-    *sp = sig;
-}
-
-template <int C, int P>
-__device__ __noinline__ void exact_gather(const GatherArgs &a, int det, int t, const QuatD &ofs, float T,
-                             float Pr) {
-    constexpr int NT = PixTraits<P>::taps;
-    double coords[4];
-    float pf[3];
-    int pix[NT][3];
-    float w[NT];
-    get_coords<C>(a.g.lut, load_quat(a.bore + 4LL * t), ofs, coords);
-    spin_factors(a.g.ncomp, coords, T, Pr, pf);
-    const int n = get_pixels<P>(a.g, coords, pix, w);
-    gather_taps<P, NT>(a, a.signal + det * a.sig_stride + t, n, pix, w, pf);
-}
-
 // One sample of the mixed-pointing fallback through the double-float
 // pointing; false (signal untouched) when its pixel is not certified.  Its
 // spin factors and terms, like the float32 tier's, are float32 evaluations
@@ -186,47 +130,6 @@ __device__ __forceinline__ bool df_gather(const GatherArgs &a, int det, int t, c
     return true;
 }
 
-// One sample of the certified float32 tier's fallback through the full
-// certified double-float pointing and certified float32 roundings of the
-// reference's float64 sums; false (signal untouched) when any of them is
-// not certain.
-template <int C, int P>
-__device__ __forceinline__ bool df_gather_cert(const GatherArgs &a, int det, int t,
-                                               const dfl (&qd)[4], float T, float Pr) {
-    constexpr int NT = PixTraits<P>::taps;
-    const double *bp = a.bore + 4LL * t;
-    const double2 lo = __ldg(reinterpret_cast<const double2 *>(bp));
-    const double2 hi = __ldg(reinterpret_cast<const double2 *>(bp) + 1);
-    dfl qb[4];
-    if (!(df_split(lo.x, qb[0]) & df_split(lo.y, qb[1]) & df_split(hi.x, qb[2]) &
-          df_split(hi.y, qb[3])))
-        return false;
-    int pix[NT][3];
-    float pf[3], w[NT];
-    int n = 0;
-    const int nc = a.g.ncomp;
-    if (!fast_pointing<C, P>(a.g, a.ft, a.fc, qb, qd, nc, T, Pr, pix, w, n, pf)) return false;
-    if (n == 0) return true;
-    float *sp = a.signal + det * a.sig_stride + t;
-    float s = *sp;
-    bool ok = true;
-#pragma unroll
-    for (int k = 0; k < NT; k++) {
-        if (k >= n || !ok) break;
-        long long off, plane;
-        const int bad = locate<P>(a.g, pix[k], &off, &plane);
-        if (bad >= 0) {
-            record_missing_tile(a.err, bad);
-            continue;
-        }
-#pragma unroll
-        for (int c = 0; c < 3; c++)
-            if (ok && c < nc) ok = fast_accum(s, __ldg(a.map + off + c * plane), pf[c], w[k]);
-    }
-    if (ok) *sp = s;
-    return ok;
-}
-
 // Compiled for 5 resident blocks per SM (at most 51 registers; mixed
 // pointing: 7), one variant per pointing mode (0 exact, 1 certified, 2
 // mixed).  The certified and mixed variants of the nearest-neighbour
@@ -240,6 +143,7 @@ __global__ void __launch_bounds__(kBlock, MixedEligible<C, P>::value && MODE == 
     __shared__ int s_queue[!kFastOK ? 1 : (kMixedOK ? 2 : 1) * (kBlock / 32) * kWarpQueue];
     __shared__ WarpPiece s_wp[kFastOK ? kBlock / 32 : 1];
     int det, t0, t1;
+    if (MODE == SO3G_POINTING_CERTIFIED && a.gate.holds()) return;
     if (!seg_piece(a.segs, a.piece, det, t0, t1)) return;
     const QuatD ofs = load_quat(a.dets + 4LL * det);
     const float T = __ldg(a.resp + 2 * det), Pr = __ldg(a.resp + 2 * det + 1);
@@ -825,6 +729,11 @@ extern "C" int so3g_proj_from_map(const so3g_pixelization *pz, const double *bor
     L.a.fast = fast_mode(pz, L.a.ft);
     L.grid = dim3((unsigned)n_det, (unsigned)((n_time + L.a.piece - 1) / L.a.piece));
     L.stream = (cudaStream_t)stream;
+    L.a.map32 = nullptr;
+    L.a.bore32 = nullptr;
+    void *cert_work = nullptr;
+    rc = cert_from_map(pz->coord_sys, pix_kind(pz), L.a, n_det, L.stream, &cert_work);
+    if (rc != 1 && rc != SO3G_OK) return rc;
     L.a.bore32 = bore_f32(pz, L.a.fast, boresight, n_time, L.stream);
     // Mixed pointing: a float32 copy of the map, pixel by pixel (over the
     // parent map when tiled), read with one 16-byte load per sample.
@@ -862,5 +771,6 @@ extern "C" int so3g_proj_from_map(const so3g_pixelization *pz, const double *bor
     rc = dispatch_cp(pz->coord_sys, pix_kind(pz), L);
     if (map32) cudaFreeAsync(map32, L.stream);
     bore_f32_free(L.a.bore32, L.stream);
+    if (cert_work) cudaFreeAsync(cert_work, L.stream);
     return rc;
 }

@@ -19,6 +19,8 @@ int after_launch(const char *what);
 // (so3g_set_chunked_min_samples); smaller calls take the per-sample float32
 // tier, whose fixed cost per call is lower.
 long long chunked_min_samples();
+// The same for the chunked certified kernels.
+long long cert_chunked_min_samples();
 // Per-device trig table (asin then atan2, 2 x kLutN float64), or NULL.
 const double *device_lut();
 

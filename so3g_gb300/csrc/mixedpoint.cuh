@@ -380,8 +380,9 @@ __device__ __forceinline__ bool mixed_zen(const DGeom &g, const MixedConst &mc,
 template <int P, bool PARENT, bool FROM_Z = false>
 __device__ __forceinline__ bool hp_pixel_f32(const DGeom &g, float lon, float elon, float z,
                                              float ez, float s, float es, int *pix) {
-    const long long nside = g.nside;
-    if (nside > (1LL << 20)) return false;
+    // nside is a power of two below 8192 (make_geom): pixel arithmetic in 32
+    // bits, divisions by shifts.
+    const int ns = (int)g.nside, lns = __ffs(ns) - 1;
     constexpr float m = 1.5f;
     // x = phi / (2 pi), wrapped into [0, 1); tt = 4 x.
     constexpr float kInv2Pi = 0.15915494f;
@@ -394,7 +395,7 @@ __device__ __forceinline__ bool hp_pixel_f32(const DGeom &g, float lon, float el
     }
     const float tt = 4.f * x, ett = 4.f * ex;
     const float za = fabsf(z);
-    const float fn = (float)(int)nside;   // nside <= 2^20: a 32-bit conversion
+    const float fn = (float)ns;
     // za <= 2/3 (the float32 2/3 is within 2e-8 of the float64 constant).
     if (!(fabsf(za - 0.6666667f) > fmaf(m, ez, 3e-8f))) return false;
     int f, ix, iy;
@@ -410,10 +411,9 @@ __device__ __forceinline__ bool hp_pixel_f32(const DGeom &g, float lon, float el
         int Jp, Jm;
         if (!(floor_cert(JP, eJ, Jp) & floor_cert(JM, eJ, Jm))) return false;
         if (Jp < 0 || Jm < 0) return false;
-        const int ns = (int)nside;
-        const int ifp = Jp / ns, ifm = Jm / ns;
-        ix = Jm - ifm * ns;
-        iy = (1 + ifp) * ns - Jp - 1;
+        const int ifp = Jp >> lns, ifm = Jm >> lns;
+        ix = Jm - (ifm << lns);
+        iy = ((1 + ifp) << lns) - Jp - 1;
         f = (ifp == ifm) ? (ifp | 4) : ((ifp < ifm) ? ifp : (ifm + 8));
     } else {
         // Polar caps: tmp = s / sqrt((1 + za) / 3), jp = tp tmp, jm = (1 - tp) tmp.
@@ -461,11 +461,10 @@ __device__ __forceinline__ bool hp_pixel_f32(const DGeom &g, float lon, float el
             return false;
     }
     const bool nest = P == PX_HP_T ? true : (g.nest != 0);
-    const long long ip = nside <= 8192 ? (long long)hp_hpd2pix32((int)nside, nest, f, ix, iy)
-                                       : hp_hpd2pix(nside, nest, f, ix, iy);
-    if (ip < 0 || ip >= g.npix) return false;
+    const int ip = hp_hpd2pix32(ns, nest, f, ix, iy);
+    if ((unsigned)ip >= (unsigned)g.npix) return false;
     if (P == PX_HP_NT || PARENT) {
-        pix[0] = (int)ip;
+        pix[0] = ip;
     } else {
         hp_tile_split(g.nppt, ip, pix[0], pix[1]);
     }

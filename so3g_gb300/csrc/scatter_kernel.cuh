@@ -25,17 +25,6 @@
 
 namespace so3g {
 
-// Internal linkage: every translation unit that includes this header gets
-// its own instantiations.
-namespace {
-
-// Resident blocks per SM the scatter kernels are compiled for (caps their
-// registers at 65536 / (kBlock * 5) = 51).  The mixed-pointing variants,
-// with more memory-latency stalls, run 7 (36 registers): measured 9 %
-// faster than 5 despite the extra spills.
-constexpr int kScatterBlocksPerSM = 5;
-constexpr int kMixedBlocksPerSM = 7;
-
 struct ScatterArgs {
     DGeom g;
     const double *bore;
@@ -54,8 +43,30 @@ struct ScatterArgs {
     FastConst fc;
     MixedConst mc;
     const float4 *bore32;   // float32 boresight (mixed pointing), or NULL
+    SkipIf gate;            // certified pointing: the kernel's gate, or none
 };
 
+// The chunked certified to_map / to_weight_map (cert_scatter.cu,
+// cert_weight.cu) over n_seg segments of up to max_len samples of n_det
+// detectors; 1 (nothing launched) where it does not apply.  On SO3G_OK the
+// chunked kernels are launched and skip, on the device, a boresight too
+// rough for them; the caller must then launch the general kernel, which
+// a.gate makes skip in the other case, and free *work (stream-ordered).
+int cert_to_map(int coord, int kind, ScatterArgs &a, int n_det, long long n_seg,
+                long long max_len, cudaStream_t st, void **work);
+int cert_to_weight_map(int coord, int kind, ScatterArgs &a, int n_det, long long n_seg,
+                       long long max_len, cudaStream_t st, void **work);
+
+// Internal linkage: every translation unit that includes this header gets
+// its own instantiations.
+namespace {
+
+// Resident blocks per SM the scatter kernels are compiled for (caps their
+// registers at 65536 / (kBlock * 5) = 51).  The mixed-pointing variants,
+// with more memory-latency stalls, run 7 (36 registers): measured 9 %
+// faster than 5 despite the extra spills.
+constexpr int kScatterBlocksPerSM = 5;
+constexpr int kMixedBlocksPerSM = 7;
 
 // Value slots: to_map slot c = component c; to_weight_map slots are the
 // upper-triangle pairs (i, j), j >= i, in row order.
@@ -373,6 +384,7 @@ __global__ void __launch_bounds__(kBlock, PointingVariant<C, P, MODE>::mixed && 
     __shared__ int s_queue[QueueInts<C, P, MODE>::value];
     __shared__ WarpPiece s_wp[kBlock / 32];
     int det, t0, t1;
+    if (MODE == SO3G_POINTING_CERTIFIED && a.gate.holds()) return;
     if (!seg_piece(a.segs, a.piece, det, t0, t1)) return;
     scatter_piece<C, P, WEIGHT, MODE>(a, det, t0, t1, s_queue, s_wp);
 }

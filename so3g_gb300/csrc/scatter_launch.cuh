@@ -73,11 +73,18 @@ int scatter_entry(const so3g_pixelization *pz, const double *bore, int32_t n_tim
     L.a.fc = make_fast_const(L.a.g);
     L.a.mc = make_mixed_const(L.a.g);
     L.a.fast = fast_mode(pz, L.a.ft);
+    L.a.bore32 = nullptr;
+    void *cert_work = nullptr;
+    rc = (WEIGHT ? cert_to_weight_map : cert_to_map)(pz->coord_sys, pix_kind(pz), L.a, n_det,
+                                                     n_seg, max_len, (cudaStream_t)stream,
+                                                     &cert_work);
+    if (rc != 1 && rc != SO3G_OK) return rc;
     L.grid = dim3((unsigned)n_seg, (unsigned)((max_len + L.a.piece - 1) / L.a.piece));
     L.stream = (cudaStream_t)stream;
     L.a.bore32 = bore_f32(pz, L.a.fast, bore, n_time, L.stream);
     rc = dispatch_cp(pz->coord_sys, pix_kind(pz), L);
     bore_f32_free(L.a.bore32, L.stream);
+    if (cert_work) cudaFreeAsync(cert_work, L.stream);
     return rc;
 }
 
