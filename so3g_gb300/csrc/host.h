@@ -61,14 +61,28 @@ int pix_kind(const so3g_pixelization *pz);
 constexpr int kBlock = 256;
 constexpr int kMinPiece = 4096;
 
-// Piece length for n_seg segments of up to max_len samples: at least
-// kMinPiece, doubled (up to 32768) while the grid would keep over 16 waves
-// of resident blocks (fewer pieces amortise the per-piece set-up), and as
+// Piece length for n_seg segments of up to max_len samples: kMinPiece,
+// doubled (up to 32768) while the grid would keep over 16 waves of resident
+// blocks (fewer pieces amortise the per-piece set-up), halved (down to one
+// round of a block) while it would not fill the GPU once (certified to_map /
+// from_map, 16 det x 4096 samples: 16 blocks of 16 serial rounds 47 / 50 us,
+// 256 of one round 19 / 19 us; 64 x 16384: 64 / 70 and 57 / 60 us), and as
 // far as needed to keep a segment within 65535 pieces.
-inline int piece_len(long long max_len, long long n_seg = 1) {
+inline int piece_len(long long max_len, long long n_seg) {
     constexpr long long kManyBlocks = 16LL * 152 * 5;
     long long p = kMinPiece;
     while (p < 32768 && n_seg * ((max_len + 2 * p - 1) / (2 * p)) >= kManyBlocks) p *= 2;
+    while (p > kBlock && n_seg * ((max_len + p - 1) / p) < 152 * 5) p /= 2;
+    while ((max_len + p - 1) / p > 65535) p *= 2;
+    return (int)p;
+}
+
+// The same for the precomputed-pointing kernels: kMinPiece, halved down to
+// the 1024 samples of a block's vectorised round while the grid would not
+// fill the GPU once.
+inline int precomp_piece_len(long long max_len, long long n_seg) {
+    long long p = kMinPiece;
+    while (p > 4 * kBlock && n_seg * ((max_len + p - 1) / p) < 152 * 5) p /= 2;
     while ((max_len + p - 1) / p > 65535) p *= 2;
     return (int)p;
 }

@@ -415,7 +415,8 @@ int point_common(PointLaunch &L, const so3g_pixelization *pz, const double *bore
     L.a.bore = bore;
     L.a.dets = dets;
     L.a.n_time = n_time;
-    L.a.piece = piece_len(n_time);
+    L.a.piece = kMinPiece;
+    while ((n_time + (long long)L.a.piece - 1) / L.a.piece > 65535) L.a.piece *= 2;
     L.grid = dim3((unsigned)n_det, (unsigned)((n_time + L.a.piece - 1) / L.a.piece));
     L.stream = (cudaStream_t)stream;
     L.what = what;

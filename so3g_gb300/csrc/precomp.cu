@@ -597,7 +597,7 @@ int so3g_precomp_to_map(const so3g_precomp_geom *g, const int32_t *pixel,
     a.sig_stride = sig_det_stride;
     a.det_weights = det_weights;
     a.segs = Segs{ranges ? ranges->seg : nullptr, n_time};
-    a.piece = piece_len(max_len);
+    a.piece = precomp_piece_len(max_len, n_seg);
     a.accum = accum;
     a.err = err;
     a.map = map->data;
@@ -623,7 +623,7 @@ int so3g_precomp_to_weight_map(const so3g_precomp_geom *g, const int32_t *pixel,
     if (n_seg <= 0 || max_len <= 0 || n_time == 0) return SO3G_OK;
     a.det_weights = det_weights;
     a.segs = Segs{ranges ? ranges->seg : nullptr, n_time};
-    a.piece = piece_len(max_len);
+    a.piece = precomp_piece_len(max_len, n_seg);
     a.accum = accum;
     a.err = err;
     a.map = map->data;
@@ -647,7 +647,7 @@ int so3g_precomp_from_map(const so3g_precomp_geom *g, const int32_t *pixel,
     a.signal_out = signal;
     a.sig_stride = sig_det_stride;
     a.segs = Segs{nullptr, n_time};
-    a.piece = piece_len(n_time);
+    a.piece = precomp_piece_len(n_time, n_det);
     a.err = err;
     a.map = map->data;
     dim3 grid((unsigned)n_det, (unsigned)((n_time + a.piece - 1) / a.piece));
