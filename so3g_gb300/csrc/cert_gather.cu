@@ -132,18 +132,17 @@ __global__ void __launch_bounds__(kBlock) k_from_map_cx_fix(const __grid_constan
                 [&](int det, int t) { cx_exact_gather<C, P>(a, det, t); });
 }
 
-constexpr int kCxGatherBlocks = 3;   // resident blocks per SM (80 registers; 4: 3 % slower)
+constexpr int kCxGatherBlocks = 6;   // resident blocks per SM (80 registers; 8: 3 % slower)
 
 template <int CL, int P, int NC>
-__global__ void __launch_bounds__(kBlock, kCxGatherBlocks)
+__global__ void __launch_bounds__(kCxBlock, kCxGatherBlocks)
     k_from_map_cx(const __grid_constant__ GatherArgs a, CxModel model, CxList left, int coord,
                   const float4 *cmap) {
     constexpr bool HP = P == PX_HP_NT || P == PX_HP_T;
     constexpr bool TILED = P == PX_FLAT_T_NN || P == PX_HP_T;
     constexpr int W = CxMap<NC, TILED>::W;
-    constexpr int kWarps = kBlock / 32;
-    __shared__ float4 s_model[kWarps][kCxGroup][kCxWords];
-    __shared__ CxWarp s_warp[kWarps];
+    __shared__ float4 s_model[kCxWarps][kCxGroup][kCxWords];
+    __shared__ CxWarp s_warp[kCxWarps];
     int det, t0, t1;
     if (a.gate.holds()) return;
     if (!seg_piece(a.segs, a.piece, det, t0, t1)) return;
@@ -176,8 +175,8 @@ __global__ void __launch_bounds__(kBlock, kCxGatherBlocks)
         }
     };
     const int j0 = t0 / kCxLen, j1 = (t1 - 1) / kCxLen + 1;
-    const int step = min(kCxGroup, (j1 - j0 + kWarps - 1) / kWarps);
-    for (int g = j0 + warp * step; g < j1; g += kWarps * step) {
+    const int step = cx_step(j1 - j0);
+    for (int g = j0 + warp * step; g < j1; g += kCxWarps * step) {
         const int nch = min(step, j1 - g);
         if (lane < nch)
             cx_setup<CL, HP, NC>(a, model.bore, coord, g + lane, n_time, qd, Pr, s_model[warp][lane]);
@@ -283,7 +282,7 @@ int cx_gather_run(const GatherArgs &a, const CxWork &w, int coord, long long npi
                                                                                 cmap);
     int rc = after_launch("from_map (map copy)");
     if (rc == SO3G_OK) {
-        k_from_map_cx<CL, P, NC><<<grid, kBlock, 0, st>>>(a, w.model, w.left, coord, cmap);
+        k_from_map_cx<CL, P, NC><<<grid, kCxBlock, 0, st>>>(a, w.model, w.left, coord, cmap);
         rc = after_launch("from_map (certified, chunked)");
     }
     cudaFreeAsync(cmap, st);

@@ -49,6 +49,8 @@ namespace {
 constexpr int kCxLen = 64;            // samples per chunk
 constexpr int kCxMid = kCxLen / 2;
 constexpr int kCxGroup = 32;          // chunks of a warp's group, one per lane
+constexpr int kCxBlock = 128;         // threads per block (its warps are independent)
+constexpr int kCxWarps = kCxBlock / 32;
 // A boresight whose residuals exceed this in more than a quarter of its
 // chunks (pointing noise of ~0.03") is not taken: the call's general kernel
 // is faster than sending most samples to the per-sample path (200 det x 500k,
@@ -637,6 +639,22 @@ __device__ __forceinline__ void cx_factor(const float4 &A, const float4 &B, floa
     S = fmaf(k, A.y, A.x);
 }
 
+// The HEALPix pixel of longitude x (error ex; < 0: none) and sin(lat) y (ey),
+// or -1 where it is not certain.  Not inlined: four copies of it in the main
+// loop made the kernel wait for instructions (400 det x 500k, nside 1024, to_map
+// and from_map: 7.5 -> 7.1 ms).
+template <int P>
+static __device__ __noinline__ int cx_hp_pixel(int nside, int nest, int npix, float x, float ex,
+                                               float y, float ey) {
+    if (!(ex >= 0.f)) return -1;
+    DGeom g;
+    g.nside = nside;
+    g.nest = nest;
+    g.npix = npix;
+    int pix[1] = {0};
+    return hp_pixel_f32<P, P == PX_HP_T, true>(g, x, ex, y, ey, 0.f, 0.f, pix) ? pix[0] : -1;
+}
+
 // One sample (k = t - mid) of a modelled chunk: pixel key (flat: iy * nx +
 // ix, of the parent map when tiled; HEALPix: the pixel), on the map or not,
 // and the spin factors of an NC-component map; false when the pixel or
@@ -654,9 +672,8 @@ __device__ __forceinline__ bool cx_sample(const float4 *w, float k, const float 
     const float y = fmaf(k, fmaf(k, fmaf(k, P1.w, P1.z), P1.y), P1.x);
     bool ok;
     if constexpr (P == PX_HP_NT || P == PX_HP_T) {
-        int pix[1] = {0};
-        ok = P2.x >= 0.f && hp_pixel_f32<P, P == PX_HP_T, true>(g, x, P2.x, y, P2.y, 0.f, 0.f, pix);
-        key = pix[0];
+        key = cx_hp_pixel<P>((int)g.nside, g.nest, (int)g.npix, x, P2.x, y, P2.y);
+        ok = key >= 0;
         on = true;
     } else {
         const float4 P3 = w[3];
@@ -805,15 +822,23 @@ __device__ __forceinline__ void cx_for_each(const CxList &list, const CxList &ne
 
 constexpr unsigned kCxFixBlocks = 152 * 8;   // of kBlock threads, striding over a list
 
+// Chunks of a warp's group for a block that has n: even shares for its warps,
+// in equal groups of at most kCxGroup, an even number (a round takes two).
+__device__ __forceinline__ int cx_step(int n) {
+    const int share = (n + kCxWarps - 1) / kCxWarps;
+    const int groups = (share + kCxGroup - 1) / kCxGroup;
+    return ((share + groups - 1) / groups + 1) & ~1;
+}
+
 // Samples per block of a call: each warp of a block takes up to kCxGroup
 // chunks at once, fewer (even) when the call would not fill the GPU twice.
 inline int cx_piece(long long n_seg, long long max_len) {
-    constexpr int kWarps = kBlock / 32;
+    constexpr long long kResident = 152 * 24;   // warps on the GPU at once
     const long long chunks = n_seg * ((max_len + kCxLen - 1) / kCxLen);
-    long long per_warp = chunks / (2LL * 152 * 4 * kWarps);
+    long long per_warp = chunks / (2 * kResident);
     per_warp = per_warp < 2 ? 2 : (per_warp > kCxGroup ? kCxGroup : per_warp & ~1LL);
-    long long p = per_warp * kWarps * kCxLen;
-    if (per_warp == kCxGroup && chunks > 16LL * 152 * 4 * kWarps * kCxGroup) p *= 2;
+    long long p = per_warp * kCxWarps * kCxLen;
+    while (per_warp == kCxGroup && p < 32768 && chunks * kCxLen > 16 * kResident / kCxWarps * p) p *= 2;
     while ((max_len + p - 1) / p > 65535) p *= 2;
     return (int)p;
 }

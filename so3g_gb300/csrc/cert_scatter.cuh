@@ -7,9 +7,8 @@
 // samples: two chunks (lanes 0-15 and 16-31), four consecutive samples per
 // lane with one 16-byte signal load, the next round's signal loaded while
 // the current one is evaluated.  A lane sums the runs of equal pixels among
-// its four samples (TwoSum: to ~2^-46) and packs them into run slots; slot j
-// of every lane is flushed with one float64 atomic per component in one
-// pass, taken only when some lane has more than j runs.  Samples the models
+// its four samples (TwoSum: to ~2^-46), one float64 atomic per run and
+// component (CxRuns).  Samples the models
 // do not certify go to a list and from there through the per-sample
 // certified path and, if need be, the float64 one (k_scatter_cx_fix).
 //
@@ -87,33 +86,31 @@ __device__ constexpr int cx_plane(int k) {
 }
 
 // Tiled maps: address and plane size of a key (flat: iy * nx + ix of the
-// parent map; HEALPix: the pixel); NULL for key < 0 and for an absent tile, which
-// is recorded.  aux: log2 of the pixels per tile (tiled HEALPix), the bits
-// of 1/nx as a float (tiled flat).
+// parent map; HEALPix: the pixel); NULL for an absent tile, which is
+// recorded.  aux: log2 of the pixels per tile (tiled HEALPix), the bits of
+// 1/nx as a float (tiled flat).
 template <int P>
 __device__ __forceinline__ double *cx_address(const ScatterArgs &a, int key, int aux, int &plane) {
-    if (key < 0) return nullptr;
+    int tile, off;
     if constexpr (P == PX_HP_T) {
-        const int tile = key >> aux;
-        const long long toff = __ldg(a.g.tile_offset + tile);
-        if (toff < 0) {
-            record_missing_tile(a.err, tile);
-            return nullptr;
-        }
-        return a.map + toff + (key & ((1 << aux) - 1));
+        tile = key >> aux;
+        off = key & ((1 << aux) - 1);
     } else {
+        // (flat_tile_tuple and locate in one: two divisions by the tile.)
         const int iy = div_small(key, a.g.nx, __int_as_float(aux)), ix = key - iy * a.g.nx;
-        int tp[3];
-        flat_tile_tuple(a.g, iy, ix, tp);
-        long long o, pl;
-        const int bad = locate<P>(a.g, tp, &o, &pl);
-        if (bad >= 0) {
-            record_missing_tile(a.err, bad);
-            return nullptr;
-        }
-        plane = (int)pl;
-        return a.map + o;
+        const int sy = div_small(iy, a.g.ty, a.g.inv_ty), sx = div_small(ix, a.g.tx, a.g.inv_tx);
+        const int y0 = sy * a.g.ty, x0 = sx * a.g.tx;
+        const int tnx = min(a.g.tx, a.g.nx - x0);
+        tile = sy * a.g.ntx + sx;
+        off = (iy - y0) * tnx + (ix - x0);
+        plane = min(a.g.ty, a.g.ny - y0) * tnx;
     }
+    const long long toff = __ldg(a.g.tile_offset + tile);
+    if (toff < 0) {
+        record_missing_tile(a.err, tile);
+        return nullptr;
+    }
+    return a.map + toff + off;
 }
 
 // The term of value k of a sample (float32 products, left to right, as
@@ -124,24 +121,22 @@ __device__ __forceinline__ float cx_value(int k, float sig, const float (&pf)[3]
     return sig * pf[k] * det_wt;
 }
 
-// Adds a run's G totals (hi + lo) of values K0.. to the map.  A lo that is
+// Adds a run's totals (hi + lo) to the map (key < 0: nothing).  A lo that is
 // NaN (an infinite hi) is left out.
-template <int P, bool WEIGHT, int NC, int K0, int G>
+template <int P, bool WEIGHT, int NC, int NV>
 __device__ __forceinline__ void cx_flush(const ScatterArgs &a, int key, int aux, int plane,
-                                         const float (&hi)[G], const float (&lo)[G]) {
-    if constexpr (P == PX_FLAT_NT_NN || P == PX_HP_NT) {
-        if (key < 0) return;
-    }
+                                         const float (&hi)[NV], const float (&lo)[NV]) {
+    if (key < 0) return;
     double *p = nullptr;
     if constexpr (P == PX_FLAT_T_NN || P == PX_HP_T) {
         p = cx_address<P>(a, key, aux, plane);
         if (!p) return;
     }
 #pragma unroll
-    for (int c = 0; c < G; c++) {
+    for (int c = 0; c < NV; c++) {
         double d = f2d(hi[c]);
         if (fabsf(lo[c]) > 0.f) d += f2d(lo[c]);
-        const int pl = cx_plane<WEIGHT, NC>(K0 + c);
+        const int pl = cx_plane<WEIGHT, NC>(c);
         // Untiled: the plane's base is the same in every lane.
         if constexpr (P == PX_FLAT_NT_NN || P == PX_HP_NT)
             atomicAdd((a.map + (long long)pl * plane) + key, d);
@@ -150,61 +145,125 @@ __device__ __forceinline__ void cx_flush(const ScatterArgs &a, int key, int aux,
     }
 }
 
-// Values K0 .. K0 + G - 1 of a lane's four samples, run by run.
-template <int P, bool WEIGHT, int NC, int K0, int G>
-__device__ __forceinline__ void cx_runs4(const ScatterArgs &a, int aux, int plane,
-                                         const int (&key)[4], const float (&sig)[4],
+// Runs a warp holds back until there are 32 to flush together: key, totals.
+// A lane's first run is flushed at once (nearly every lane has one), its
+// others (about half the lanes have one) go here: 1.6 full passes of atomics
+// per 128 samples where flushing slot by slot took 2.2 part-filled ones, one
+// copy of the flush code instead of four.
+template <int NV>
+struct CxRuns {
+    // Most runs a round may add (else it is added term by term); six values
+    // a run leave room for fewer (20 warps on an SM).
+    static constexpr int more = NV > 3 ? 48 : 64;
+    static constexpr int W = (1 + 2 * NV + 3) / 4;
+    float4 rec[W][more + 32];
+};
+
+template <int NV>
+__device__ __forceinline__ void cx_run_put(CxRuns<NV> &rb, int pos, int key, const float (&hi)[NV],
+                                           const float (&lo)[NV]) {
+    constexpr int W = CxRuns<NV>::W;
+    float x[4 * W];
+#pragma unroll
+    for (int k = 0; k < 4 * W; k++)
+        x[k] = k == 0 ? __int_as_float(key)
+                      : (k <= NV ? hi[k <= NV ? k - 1 : 0]
+                                 : (k <= 2 * NV ? lo[k <= 2 * NV && k > NV ? k - 1 - NV : 0] : 0.f));
+#pragma unroll
+    for (int w = 0; w < W; w++)
+        rb.rec[w][pos] = make_float4(x[4 * w], x[4 * w + 1], x[4 * w + 2], x[4 * w + 3]);
+}
+
+// Flushes the last min(32, n) runs held back, one per lane.
+template <int P, bool WEIGHT, int NC, int NV>
+__device__ __forceinline__ void cx_run_flush(const ScatterArgs &a, CxRuns<NV> &rb, int n, int aux,
+                                             int plane) {
+    constexpr int W = CxRuns<NV>::W;
+    const int i = n - 1 - (int)(threadIdx.x & 31);
+    if (i < 0) return;
+    float x[4 * W], hi[NV], lo[NV];
+#pragma unroll
+    for (int w = 0; w < W; w++) {
+        const float4 v = rb.rec[w][i];
+        x[4 * w] = v.x;
+        x[4 * w + 1] = v.y;
+        x[4 * w + 2] = v.z;
+        x[4 * w + 3] = v.w;
+    }
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+        hi[k] = x[1 + k];
+        lo[k] = x[1 + NV + k];
+    }
+    cx_flush<P, WEIGHT, NC, NV>(a, __float_as_int(x[0]), aux, plane, hi, lo);
+}
+
+// The runs of equal pixels among a lane's four samples: the first flushed,
+// the others held back (nr: runs held back so far; flushed down to fewer
+// than 32).  False (nothing done) when the round has too many further
+// runs.  All lanes must call.
+template <int P, bool WEIGHT, int NC, int NV>
+__device__ __forceinline__ bool cx_runs4(const ScatterArgs &a, CxRuns<NV> &rb, int &nr, int aux,
+                                         int plane, const int (&key)[4], const float (&sig)[4],
                                          const float (&pf)[4][3], float det_wt) {
-    float v[4][G], lo[4][G];
+    const bool h1 = key[1] != key[0], h2 = key[2] != key[1], h3 = key[3] != key[2];
+    const bool p1 = h1 & (key[1] >= 0), p2 = h2 & (key[2] >= 0), p3 = h3 & (key[3] >= 0);
+    const int n = (int)p1 + (int)p2 + (int)p3;
+    const unsigned b0 = __ballot_sync(kFull, n & 1), b1 = __ballot_sync(kFull, n & 2);
+    const int total = __popc(b0) + 2 * __popc(b1);
+    if (total > CxRuns<NV>::more) return false;
+    float v[4][NV], lo[4][NV];
 #pragma unroll
     for (int j = 0; j < 4; j++)
 #pragma unroll
-        for (int c = 0; c < G; c++) {
-            v[j][c] = cx_value<WEIGHT, NC>(K0 + c, sig[j], pf[j], det_wt);
+        for (int c = 0; c < NV; c++) {
+            v[j][c] = cx_value<WEIGHT, NC>(c, sig[j], pf[j], det_wt);
             lo[j][c] = 0.f;
         }
-    const bool h1 = key[1] != key[0], h2 = key[2] != key[1], h3 = key[3] != key[2];
+    // Right to left: v[i] + lo[i] becomes the total of the run from i on.
 #pragma unroll
-    for (int c = 0; c < G; c++) {
+    for (int c = 0; c < NV; c++) {
         float e;
         if (!h3) { two_sum(v[2][c], v[3][c], v[2][c], e); lo[2][c] = e; }
         if (!h2) { two_sum(v[1][c], v[2][c], v[1][c], e); lo[1][c] = lo[2][c] + e; }
         if (!h1) { two_sum(v[0][c], v[1][c], v[0][c], e); lo[0][c] = lo[1][c] + e; }
     }
-    // Slots 1 and 2: the first and second heads among samples 1..3; slot
-    // 3: sample 3 when all three are heads.
-    const int nruns = 1 + h1 + h2 + h3;
-    float s1[G], l1[G], s2[G], l2[G];
-#pragma unroll
-    for (int c = 0; c < G; c++) {
-        s1[c] = h1 ? v[1][c] : (h2 ? v[2][c] : v[3][c]);
-        l1[c] = h1 ? lo[1][c] : (h2 ? lo[2][c] : lo[3][c]);
-        s2[c] = (h1 && h2) ? v[2][c] : v[3][c];
-        l2[c] = (h1 && h2) ? lo[2][c] : lo[3][c];
+    if (total) {
+        const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
+        int pos = nr + __popc(b0 & lt) + 2 * __popc(b1 & lt);
+        if (p1) cx_run_put<NV>(rb, pos, key[1], v[1], lo[1]);
+        pos += p1;
+        if (p2) cx_run_put<NV>(rb, pos, key[2], v[2], lo[2]);
+        pos += p2;
+        if (p3) cx_run_put<NV>(rb, pos, key[3], v[3], lo[3]);
+        nr += total;
+        __syncwarp();
     }
-    const int k1 = h1 ? key[1] : (h2 ? key[2] : key[3]);
-    const int k2 = (h1 && h2) ? key[2] : key[3];
-    cx_flush<P, WEIGHT, NC, K0, G>(a, key[0], aux, plane, v[0], lo[0]);
-    if (__any_sync(kFull, nruns > 1) && nruns > 1)
-        cx_flush<P, WEIGHT, NC, K0, G>(a, k1, aux, plane, s1, l1);
-    if (__any_sync(kFull, nruns > 2) && nruns > 2)
-        cx_flush<P, WEIGHT, NC, K0, G>(a, k2, aux, plane, s2, l2);
-    if (__any_sync(kFull, nruns > 3) && nruns > 3)
-        cx_flush<P, WEIGHT, NC, K0, G>(a, key[3], aux, plane, v[3], lo[3]);
+    cx_flush<P, WEIGHT, NC, NV>(a, key[0], aux, plane, v[0], lo[0]);
+    while (nr >= 32) {
+        cx_run_flush<P, WEIGHT, NC, NV>(a, rb, nr, aux, plane);
+        nr -= 32;
+        __syncwarp();
+    }
+    return true;
 }
 
-// Resident blocks per SM: 3 leave 80 registers; 4 (64, more spills) took 5 %
-// longer in to_map, 5 another 15 %.
-constexpr int kCxScatterBlocks = 3;
+// Resident blocks per SM: 24 warps with 80 registers (to_map; 32 warps with
+// 64, more spills, took 5 % longer, 40 another 15 %), 20 (to_weight_map, whose
+// held-back runs take more shared memory).
+template <bool WEIGHT>
+struct CxScatterBlocks {
+    static constexpr int value = WEIGHT ? 4 : 5;
+};
 
 template <int CL, int P, bool WEIGHT, int NC>
-__global__ void __launch_bounds__(kBlock, kCxScatterBlocks)
+__global__ void __launch_bounds__(kCxBlock, CxScatterBlocks<WEIGHT>::value)
     k_scatter_cx(const __grid_constant__ ScatterArgs a, CxModel model, CxList left, int coord) {
     constexpr bool HP = P == PX_HP_NT || P == PX_HP_T;
     constexpr int NV = WEIGHT ? NC * (NC + 1) / 2 : NC;
-    constexpr int kWarps = kBlock / 32;
-    __shared__ float4 s_model[kWarps][kCxGroup][kCxWords];
-    __shared__ CxWarp s_warp[kWarps];
+    __shared__ float4 s_model[kCxWarps][kCxGroup][kCxWords];
+    __shared__ CxWarp s_warp[kCxWarps];
+    __shared__ CxRuns<NV> s_runs[kCxWarps];
     int det, t0, t1;
     if (a.gate.holds()) return;
     if (!seg_piece(a.segs, a.piece, det, t0, t1)) return;
@@ -262,9 +321,10 @@ __global__ void __launch_bounds__(kBlock, kCxScatterBlocks)
             }
         }
     };
+    int nr = 0;   // runs held back
     const int j0 = t0 / kCxLen, j1 = (t1 - 1) / kCxLen + 1;
-    const int step = min(kCxGroup, (j1 - j0 + kWarps - 1) / kWarps);
-    for (int g = j0 + warp * step; g < j1; g += kWarps * step) {
+    const int step = cx_step(j1 - j0);
+    for (int g = j0 + warp * step; g < j1; g += kCxWarps * step) {
         const int nch = min(step, j1 - g);
         if (lane < nch)
             cx_setup<CL, HP, NC>(a, model.bore, coord, g + lane, n_time, qd, Pr, s_model[warp][lane]);
@@ -308,12 +368,10 @@ __global__ void __launch_bounds__(kBlock, kCxScatterBlocks)
                     }
             }
             const float size = WEIGHT ? 1.f : fabsf(sg[0]) + fabsf(sg[1]) + fabsf(sg[2]) + fabsf(sg[3]);
-            const bool by_run = a.accum == SO3G_ACCUM_WARP_RUNS && __all_sync(kFull, size < lim);
-            if (by_run) {
-                cx_runs4<P, WEIGHT, NC, 0, (NV < 3 ? NV : 3)>(a, aux, plane, key, sg, pf, det_wt);
-                if constexpr (NV > 3)
-                    cx_runs4<P, WEIGHT, NC, 3, NV - 3>(a, aux, plane, key, sg, pf, det_wt);
-            } else {
+            const bool by_run =
+                a.accum == SO3G_ACCUM_WARP_RUNS && __all_sync(kFull, size < lim) &&
+                cx_runs4<P, WEIGHT, NC, NV>(a, s_runs[warp], nr, aux, plane, key, sg, pf, det_wt);
+            if (!by_run) {
 #pragma unroll 1
                 for (int i = 0; i < 4; i++) {
                     const int kk = i == 0 ? key[0] : (i == 1 ? key[1] : (i == 2 ? key[2] : key[3]));
@@ -327,7 +385,7 @@ __global__ void __launch_bounds__(kBlock, kCxScatterBlocks)
                         v[k] = cx_value<WEIGHT, NC>(k, s, f, det_wt);
                         z[k] = 0.f;
                     }
-                    cx_flush<P, WEIGHT, NC, 0, NV>(a, kk, aux, plane, v, z);
+                    cx_flush<P, WEIGHT, NC, NV>(a, kk, aux, plane, v, z);
                 }
             }
             if (__any_sync(kFull, f4 != 0u) && cx_enqueue(cw, f4, tq) >= 32)
@@ -335,6 +393,7 @@ __global__ void __launch_bounds__(kBlock, kCxScatterBlocks)
         }
         __syncwarp();
     }
+    if (nr > 0) cx_run_flush<P, WEIGHT, NC, NV>(a, s_runs[warp], nr, aux, plane);
     cx_append(cw, left, det, over);
 }
 
@@ -351,9 +410,9 @@ template <int CL, int P, bool WEIGHT>
 int cx_scatter_launch(const ScatterArgs &a, const CxWork &w, int coord, dim3 grid,
                       cudaStream_t st) {
     switch (a.g.ncomp) {
-    case 1: k_scatter_cx<CL, P, WEIGHT, 1><<<grid, kBlock, 0, st>>>(a, w.model, w.left, coord); break;
-    case 2: k_scatter_cx<CL, P, WEIGHT, 2><<<grid, kBlock, 0, st>>>(a, w.model, w.left, coord); break;
-    default: k_scatter_cx<CL, P, WEIGHT, 3><<<grid, kBlock, 0, st>>>(a, w.model, w.left, coord); break;
+    case 1: k_scatter_cx<CL, P, WEIGHT, 1><<<grid, kCxBlock, 0, st>>>(a, w.model, w.left, coord); break;
+    case 2: k_scatter_cx<CL, P, WEIGHT, 2><<<grid, kCxBlock, 0, st>>>(a, w.model, w.left, coord); break;
+    default: k_scatter_cx<CL, P, WEIGHT, 3><<<grid, kCxBlock, 0, st>>>(a, w.model, w.left, coord); break;
     }
     const int rc = after_launch(WEIGHT ? "to_weight_map (certified, chunked)"
                                        : "to_map (certified, chunked)");

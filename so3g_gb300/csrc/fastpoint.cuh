@@ -130,8 +130,10 @@ __device__ __forceinline__ dfl df_dot(const dfl (&x)[N], const dfl (&y)[N]) {
     return fast_two_sum(s, e);
 }
 
-// Double-float from a double through the conversion instructions.
-__device__ __forceinline__ dfl df_from_double(double x) {
+// Double-float from a double through the conversion instructions (rarely
+// taken; inlined, they are issued for every value and only the selection
+// depends on it, and each takes the float64 pipe ~20 cycles a warp).
+static __device__ __noinline__ dfl df_from_double(double x) {
     float hi = __double2float_rn(x);
     float lo = __double2float_rn(x - (double)hi);
     return dfl{hi, lo};
