@@ -25,10 +25,11 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-fmad=false", "-Xcompiler", "-f
               "-Xptxas", "-warn-spills"]
 UNITS = ["api.cu", "pointing.cu", "scatter.cu", "scatter_weight.cu", "gather.cu", "precomp.cu",
          "noalloc.cu", "batch.cu", "batch_weight.cu", "sightline.cu", "ranges.cu",
-         "cert_scatter.cu", "cert_weight.cu", "cert_gather.cu"]
+         "cert_scatter.cu", "cert_weight.cu", "cert_gather.cu", "bilinear_gather.cu"]
 HEADERS = ["device.cuh", "host.h", "scatter_kernel.cuh", "scatter_launch.cuh", "batch_launch.cuh",
            "fastpoint.cuh", "mixedpoint.cuh", "mixed_launch.cuh", "mx_common.cuh", "interp_point.cuh",
-           "cert_point.cuh", "cert_scatter.cuh", "gather_kernel.cuh"]
+           "cert_point.cuh", "cert_scatter.cuh", "gather_kernel.cuh",
+           "cert_map.cuh"]
 
 
 def nvcc():

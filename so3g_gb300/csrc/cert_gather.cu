@@ -13,89 +13,12 @@
 // samples: 30.9 -> 8.4 ms (of which 0.9 ms the fallback).
 
 #include "cert_point.cuh"
+#include "cert_map.cuh"
 #include "gather_kernel.cuh"
 
 namespace so3g {
 
 namespace {
-
-// float4 words per pixel of the map copy: the pairs (h, l), for a tiled map
-// followed by the tile's presence in the last word's .w.
-template <int NC, bool TILED>
-struct CxMap {
-    static constexpr int W = TILED ? (NC == 1 ? 1 : 2) : (NC + 1) / 2;
-};
-
-// The copy, over the parent map's pixels when tiled: h = +-0 for m = +-0,
-// NaN where m is not finite or outside df_split's range (such a sample goes
-// to the float64 path).
-template <int P, int NC>
-__global__ void k_cx_map(DGeom g, const double *map, long long npix, float4 *out) {
-    constexpr bool TILED = P == PX_FLAT_T_NN || P == PX_HP_T;
-    constexpr int W = CxMap<NC, TILED>::W;
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npix) return;
-    long long off = i, plane = npix;
-    bool present = true;
-    if constexpr (TILED) {
-        int pix[3];
-        if (P == PX_HP_T) {
-            hp_tile_split(g.nppt, i, pix[0], pix[1]);
-            pix[2] = 0;
-        } else {
-            const int gy = (int)(i / g.nx), gx = (int)(i - (long long)gy * g.nx);
-            flat_tile_tuple(g, gy, gx, pix);
-        }
-        present = locate<P>(g, pix, &off, &plane) < 0;
-    }
-    float hl[4 * W];
-#pragma unroll
-    for (int k = 0; k < 4 * W; k++) hl[k] = 0.f;
-    if (present) {
-#pragma unroll
-        for (int c = 0; c < NC; c++) {
-            const double m = __ldg(map + off + c * plane);
-            const unsigned mh = (unsigned)__double2hiint(m);
-            float h = __int_as_float(0x7fc00000), l = 0.f;
-            if (((mh & 0x7fffffffu) | (unsigned)__double2loint(m)) == 0u) {
-                h = __uint_as_float(mh & 0x80000000u);
-            } else {
-                dfl d;
-                if (df_split(m, d)) {
-                    h = d.hi;
-                    l = d.lo;
-                }
-            }
-            hl[2 * c] = h;
-            hl[2 * c + 1] = l;
-        }
-    }
-    if (TILED) hl[4 * W - 1] = present ? 1.f : 0.f;
-#pragma unroll
-    for (int w = 0; w < W; w++)
-        out[i * W + w] = make_float4(hl[4 * w], hl[4 * w + 1], hl[4 * w + 2], hl[4 * w + 3]);
-}
-
-// sig + m * pf rounded to float32 as the reference's `*sig += map * pf`, m =
-// h + l from the map copy; false when that rounding is not certain.  S + L
-// is the double-float sum (S = fl(sig + h pf)), within e of the reference's
-// float64 sum (as fast_accum).
-__device__ __forceinline__ bool cx_accum(float &sig, float h, float l, float pf) {
-    const float p = h * pf;
-    const float pe = fmaf(l, pf, fmaf(h, pf, -p));
-    float S, x;
-    two_sum(sig, p, S, x);
-    const float L = x + pe, e = 5e-13f * (fabsf(p) + fabsf(sig));
-    float r = S + (L + e);
-    bool ok = (r == S + (L - e)) & (fabsf(r) > 1e-30f);
-    if (!ok && (h == 0.f || (pf == 0.f && h == h))) {
-        // An exact zero with the product's sign (as fast_accum).
-        r = sig + __int_as_float((__float_as_int(h) ^ __float_as_int(pf)) & 0x80000000);
-        ok = true;
-    }
-    if (ok) sig = r;
-    return ok;
-}
 
 // One sample the models left: the certified double-float pointing (false:
 // not certain), the float64 pointing.

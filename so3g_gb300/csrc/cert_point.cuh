@@ -91,6 +91,19 @@ struct CxModel {
 // sin(lat), with xb = yb = 0 and hx, hy their error bounds (hx < 0: not
 // modelled).  g0 + k g1: the gradient of phi, per residual unit.
 constexpr int kCxWords = 9;
+// The bilinear form (TAN, ZEA, SIN; thirteen words) holds the pixel
+// coordinates as the spin factors are, exact part plus correction, and their
+// gradients per residual unit:
+//   0: fx0 fx1 lx0 lx1   1: x2 x3 x4 e   2: fy0 fy1 ly0 ly1   3: xb yb mid flag
+//   4 .. 8: as above   9: y2 y3 y4 -   10, 11, 12: jx0 jx1 jy0 jy1 for the
+//   residual's components x, y, z (each g0 + k g1)
+// with the unmodelled chunks' e = -1 (pixel bound kCxBlPix).
+constexpr int kCxBlWords = 13;
+// Bilinear weights need the fraction of a pixel to float32 accuracy: a chunk
+// whose pixel coordinates are not within this of the reference's goes to the
+// per-sample path (the bound is several times the error; a float32 weight is
+// good to 3e-8).
+constexpr float kCxBlPix = 2.5e-7f;
 // 1.5 x 2^23: x + kCxMagic is x rounded to the nearest integer (|x| < 2^21),
 // its low bits that integer -- one addition instead of a floor and a
 // conversion on the slow conversion pipe.
@@ -303,14 +316,53 @@ __device__ __forceinline__ float cx_gradient(const float (&A)[4], const float (&
     return cf_abs(k);
 }
 
+// Gradient of the zenithal pixel coordinates (X, Y) with respect to rho, at A
+// = q q_det, per unit of rotation: with W = alpha conj(beta) = (Y - i X) / G,
+// G = g(n) 2, rho' = (x, y, z): dW = (y - i x) alpha^2 - (y + i x)
+// conj(beta)^2, dn = -2 Re((y + i x) conj(alpha beta)).
+__device__ __forceinline__ void cx_pixel_gradient(int coord, const float (&A)[4],
+                                                  const float (&d)[4], float (&gx)[3],
+                                                  float (&gy)[3]) {
+    const cf al{A[0], A[3]}, be{A[2], A[1]}, bc{A[2], -A[1]};
+    const cf a2 = al * al, b2 = bc * bc, v = al * be, W = al * bc;
+    const float n = al.r * al.r + al.i * al.i;
+    float G = 2.f, dG = 0.f;   // dG / dn
+    if (coord == SO3G_COORD_TAN) {
+        const float r = rcp_approx(2.f * n - 1.f);
+        G = 2.f * r;
+        dG = -4.f * r * r;
+    } else if (coord == SO3G_COORD_ZEA) {
+        const float r = rsqrtf(n);
+        G = 2.f * r;
+        dG = -r * r * r;
+    }
+    // y: dW = a2 - b2, dn = -2 Re v;  x: dW = -i (a2 + b2), dn = -2 Im v.
+    const cf jy = G * (a2 - b2) + (-2.f * v.r * dG) * W;
+    const cf sp = a2 + b2;
+    const cf jx = G * cf{sp.i, -sp.r} + (-2.f * v.i * dG) * W;
+    // (d(Y - i X): Y the real part, X minus the imaginary one); components
+    // along x and y of the detector's frame, turned to the boresight's.
+    const float in[2][2] = {{-jx.i, -jy.i}, {jx.r, jy.r}};
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+        const float x = in[c][0], y = in[c][1];
+        const float tx = -2.f * d[3] * y, ty = 2.f * d[3] * x, tz = 2.f * (d[1] * y - d[2] * x);
+        float(&g)[3] = c == 0 ? gx : gy;
+        g[0] = x + d[0] * tx + d[2] * tz - d[3] * ty;
+        g[1] = y + d[0] * ty + d[3] * tx - d[1] * tz;
+        g[2] = d[0] * tz + d[1] * ty - d[2] * tx;
+    }
+}
+
 // The model of chunk j for a detector (double-float qd), into w (kCxWords
-// words).
-template <int CL, bool HP, int NC, class Args>
+// words; BL: the bilinear form, kCxBlWords).
+template <int CL, bool HP, int NC, bool BL = false, class Args>
 __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int coord, int j,
                                          int n_time, const dfl (&qd)[4], float Pr, float4 *w) {
     constexpr bool SPIN = NC > 1;
     constexpr float u = kU;
     const int mid = cx_mid(j, n_time);
+    if (BL) w[1] = make_float4(0.f, 0.f, 0.f, -1.f);
     w[2] = make_float4(-1.f, -1.f, 0.f, 0.f);
     w[3] = make_float4(0.f, 0.f, __int_as_float(mid), 0.f);
     const CxBore &cb = cxb[j];
@@ -373,6 +425,7 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
     float lutx = 0.f, luty = 0.f;    // the tables' errors at both ends
     float zz;                        // |z1|^2 of alpha and beta
     float gerr;                      // gradient of phi: error of its linear form
+    cf x4{0.f, 0.f};                 // BL: the u^4 coefficient of Y - i X
     if constexpr (CL == CX_CAR) {
         if (!(be2 > 0.004f)) return;
         const float ib = rcp_approx(be2);
@@ -492,8 +545,36 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         const float k0 = cf_abs(b0), k1 = 0.5f * cf_abs(b1), k2 = 0.25f * cf_abs(b2),
                     k3 = 0.125f * cf_abs(b3), k4 = 0.0625f * cf_abs(cf{A4[2], A4[1]});
         const float h2 = h * h;
-        tx = ty = g * (4.f * (k0 * h2 * h2 + k1 * h2 * h + k2 * h2 + k3 * h) + 1.2f * k4) *
-                      1.2f + 1e-12f;
+        if constexpr (BL) {
+            // (One order more.)
+            const cf b4{A4[2], -A4[1]};
+            cf e4;
+            if (coord == SO3G_COORD_TAN) {
+                const float ic = rcp_approx(2.f * al2 - 1.f), f = 2.f * al2 * ic;
+                const float q1 = 2.f * la.l1.r, q2 = 2.f * la.l2.r, q3 = 2.f * la.l3.r,
+                            q4 = 2.f * la.l4.r;
+                const float x1 = f * q1, x2 = f * (q2 + 0.5f * q1 * q1),
+                            x3 = f * (q3 + q1 * q2 + (1.f / 6.f) * q1 * q1 * q1),
+                            x4_ = f * (q4 + q1 * q3 + 0.5f * q2 * q2 + 0.5f * q1 * q1 * q2 +
+                                       (1.f / 24.f) * q1 * q1 * q1 * q1);
+                const float g1 = -x1, g2 = x1 * x1 - x2, g3 = 2.f * x1 * x2 - x3 - x1 * x1 * x1,
+                            g4 = 2.f * x1 * x3 - x4_ + x2 * x2 - 3.f * x1 * x1 * x2 +
+                                 x1 * x1 * x1 * x1;
+                e4 = cf{A4[0], A4[3]} * inv_a + g1 * z3 + g2 * z2 + g3 * z1 + cf{g4, 0.f};
+            } else if (coord == SO3G_COORD_ZEA) {
+                const float t1 = la.l1.i, t2 = la.l2.i, t3 = la.l3.i, t4 = la.l4.i;
+                e4 = cf{-t1 * t3 - 0.5f * t2 * t2 + (1.f / 24.f) * t1 * t1 * t1 * t1,
+                        t4 - 0.5f * t1 * t1 * t2};
+            } else {
+                e4 = cf{A4[0], A4[3]} * inv_a;
+            }
+            x4 = s * (b4 + e1 * b3 + e2 * b2 + e3 * b1 + e4 * b0);
+            tx = ty = g * 5.f * h * (k0 * h2 * h2 + k1 * h2 * h + k2 * h2 + k3 * h + 1.2f * k4) *
+                          1.2f + 1e-13f;
+        } else {
+            tx = ty = g * (4.f * (k0 * h2 * h2 + k1 * h2 * h + k2 * h2 + k3 * h) + 1.2f * k4) *
+                          1.2f + 1e-12f;
+        }
     }
     // Pixel coordinates: the coefficients' float32 errors (24u of the terms'
     // sizes, of which cx1 .. carry products of at most a few factors), the
@@ -531,10 +612,83 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         ey = 1.5f * (ey + 2.f * kEpsPix + 2.f * u);
     }
     constexpr float s1 = 1.f / 64.f, s2 = s1 * s1, s3 = s2 * s1, s4 = s2 * s2;
+    if constexpr (BL) {
+        // X', Y' at the middle in double-float: Y' - i X' = s b1 + e1 (Y0 - i
+        // X0), s = 2 g alpha_0, b1 = conj(beta_1), e1 = i Im z1 (ZEA), z1 (SIN)
+        // or z1 - 4 n Re(z1) / (2n - 1) (TAN), z1 = alpha_1 / alpha_0.
+        dfl p, r, s, t;
+        {
+            const float4 h = __ldg(&cb.a1_hi), l = __ldg(&cb.a1_lo);
+            const dfl q[4] = {{h.x, l.x}, {h.y, l.y}, {h.z, l.z}, {h.w, l.w}};
+            df_qmul(q, qd, p, r, s, t);
+        }
+        const dfl n = df_dot<2>({qa, qe}, {qa, qe}), rn = df_recip(n);
+        const dfl ei = df_mul(df_dot<2>({t, p}, {qa, df_neg(qe)}), rn);
+        dfl er = df_mul(df_dot<2>({p, t}, {qa, qe}), rn), G{2.f, 0.f};
+        if (coord == SO3G_COORD_TAN) {
+            const dfl rc = df_recip(df_sub(df_mulf(n, 2.f), dfl{1.f, 0.f}));
+            G = df_mulf(rc, 2.f);
+            er = df_sub(er, df_mul(df_mulf(df_mul(n, rc), 4.f), er));
+        } else if (coord == SO3G_COORD_ZEA) {
+            const float r0 = sqrtf(n.hi);
+            const dfl sq = fast_two_sum(r0, (fmaf(-r0, r0, n.hi) + n.lo) / (2.f * r0));
+            G = df_mulf(df_recip(sq), 2.f);
+            er = dfl{0.f, 0.f};
+        }
+        const dfl yr = df_mul(G, df_dot<2>({qa, qe}, {s, r}));
+        const dfl yi = df_mul(G, df_dot<2>({qe, qa}, {s, df_neg(r)}));
+        const dfl Y1 = df_add(yr, df_dot<2>({er, ei}, {Y0, X0}));
+        const dfl X1 = df_sub(df_dot<2>({er, ei}, {X0, df_neg(Y0)}), yi);
+        const dfl xa = df_add(df_mul(X0, a.fc.inv_cdx), a.fc.off_x);
+        const dfl ya = df_add(df_mul(Y0, a.fc.inv_cdy), a.fc.off_y);
+        dfl fx, fy;
+        df_floor(xa, fx);
+        df_floor(ya, fy);
+        fx = df_sub(fx, dfl{0.5f, 0.f});
+        fy = df_sub(fy, dfl{0.5f, 0.f});
+        // Exact parts in multiples of 2^-17 pixel (below 64 pixels in all).
+        constexpr float cst = 96.f;
+        const dfl vx = df_mulf(df_mul(X1, a.fc.inv_cdx), s1), vy = df_mulf(df_mul(Y1, a.fc.inv_cdy), s1);
+        const float fx0 = (fx.hi + cst) - cst, fx1 = (vx.hi + cst) - cst;
+        const float fy0 = (fy.hi + cst) - cst, fy1 = (vy.hi + cst) - cst;
+        const float x2 = cx2 * icx * s2, x3 = cx3 * icx * s3, x4p = -x4.i * icx * s4;
+        const float y2 = cy2 * icy * s2, y3 = cy3 * icy * s3, y4p = x4.r * icy * s4;
+        // Errors: the terms left out, the corrections' float32 roundings and
+        // those of the coefficients (12u of their terms), the residual's
+        // second order and quantisation, its gradient's linear form.
+        const float cor = 1024.f * (fabsf(cx2 * icx) + fabsf(cy2 * icy)) * s2 +
+                          32768.f * (fabsf(cx3 * icx) + fabsf(cy3 * icy)) * s3 + 2e-4f;
+        const float ai = fmaxf(aix, aiy);
+        const float eb = tx * ai + 12.f * u * cor + 3e-12f * rx * ai +
+                         (lsb > 0.f ? rx * ai * (E * (16.f * E + 2.f * zz + 32.f * u) + 2.f * lsb)
+                                    : rx * ai * E);
+        if (!(eb < kCxBlPix && (sx * aix + 1.f) < 60.f && (sy * aiy + 1.f) < 60.f)) return;
+        w[0] = make_float4(fx0, fx1, (fx.hi - fx0) + fx.lo, (vx.hi - fx1) + vx.lo);
+        w[1] = make_float4(x2, x3, x4p, -1.f);
+        w[2] = make_float4(fy0, fy1, (fy.hi - fy0) + fy.lo, (vy.hi - fy1) + vy.lo);
+        w[9] = make_float4(y2, y3, y4p, 0.f);
+        if (lsb > 0.f) {
+            float N0[4], N1[4], gx0[3], gx1[3], gy0[3], gy1[3];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                N0[c] = A[c] - 0.5f * A1[c] + 0.25f * A2[c];
+                N1[c] = A[c] + 0.5f * A1[c] + 0.25f * A2[c];
+            }
+            cx_pixel_gradient(coord, N0, d32, gx0, gy0);
+            cx_pixel_gradient(coord, N1, d32, gx1, gy1);
+            const float hx = 0.5f * lsb * icx, hy = 0.5f * lsb * icy;
+            const float dx = lsb * s1 * icx, dy = lsb * s1 * icy;
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+                w[10 + c] = make_float4((gx0[c] + gx1[c]) * hx, (gx1[c] - gx0[c]) * dx,
+                                        (gy0[c] + gy1[c]) * hy, (gy1[c] - gy0[c]) * dy);
+        }
+    } else {
     w[0] = make_float4(xf, cx1 * icx * s1, cx2 * icx * s2, cx3 * icx * s3);
     w[1] = make_float4(yf, cy1 * icy * s1, cy2 * icy * s2, cy3 * icy * s3);
+    }
     float e = 0.f;
-    bool flag = false;
+    bool flag = BL && lsb > 0.f;
     if constexpr (SPIN) {
         // The spin factors at the middle, F1 + i F2 = P v^2 / D, and phi's
         // derivative there, 2 (Im(alpha_1 conj(alpha_0)) / |alpha_0|^2 + ...
@@ -627,7 +781,8 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         }
         if (!fine) e = __int_as_float(0x7f800000);   // never certain
     }
-    w[2] = make_float4(HP ? ex : 0.5f - ex, HP ? ey : 0.5f - ey, e, 0.f);
+    if constexpr (BL) w[1].w = e;
+    else w[2] = make_float4(HP ? ex : 0.5f - ex, HP ? ey : 0.5f - ey, e, 0.f);
     w[3] = make_float4(__int_as_float(xb), __int_as_float(yb), __int_as_float(mid),
                        flag ? 1.f : 0.f);
 }

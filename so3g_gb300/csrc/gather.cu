@@ -25,19 +25,6 @@ namespace {
 // copy spans the parent map (16 bytes per pixel), present tiles or not.
 constexpr long long kMap32TiledMaxPixels = 1LL << 28;
 
-// Index of a located sample's pixel in the float32 map copy: its element
-// offset for an untiled map; for a tiled map its pixel in the parent map
-// (flat: row-major over (ny, nx); HEALPix: the NEST index tile * nppt + sub).
-template <int P>
-__device__ __forceinline__ long long map32_index(const DGeom &g, const int *pix, long long off) {
-    if (P == PX_FLAT_T_NN || P == PX_FLAT_T_BL) {
-        const int t = pix[0], row = div_small(t, g.ntx, g.inv_ntx), col = t - row * g.ntx;
-        return (long long)(row * g.ty + pix[1]) * g.nx + (long long)col * g.tx + pix[2];
-    }
-    if (P == PX_HP_T) return (long long)pix[0] * g.nppt + pix[1];
-    return off;
-}
-
 // Tile tuple of a parent-map pixel in the float32 tier's PARENT form.
 template <int P>
 __device__ __forceinline__ void parent_to_tile(const DGeom &g, const int *par, int *tp) {
@@ -82,54 +69,6 @@ __global__ void k_map_f32(const double *map, int nc, long long npix, float4 *out
     out[i] = make_float4(v[0], v[1], v[2], 0.f);
 }
 
-// One sample of the mixed-pointing fallback through the double-float
-// pointing; false (signal untouched) when its pixel is not certified.  Its
-// spin factors and terms, like the float32 tier's, are float32 evaluations
-// (the mixed-precision contract).
-template <int C, int P>
-__device__ __forceinline__ bool df_gather(const GatherArgs &a, int det, int t, const dfl (&qd)[4], float T,
-                          float Pr) {
-    constexpr int NT = PixTraits<P>::taps;
-    const double *bp = a.bore + 4LL * t;
-    const double2 lo = __ldg(reinterpret_cast<const double2 *>(bp));
-    const double2 hi = __ldg(reinterpret_cast<const double2 *>(bp) + 1);
-    dfl qb[4];
-    if (!(df_split(lo.x, qb[0]) & df_split(lo.y, qb[1]) & df_split(hi.x, qb[2]) &
-          df_split(hi.y, qb[3])))
-        return false;
-    int pix[NT][3];
-    float pf[3], w[NT];
-    int n = 0;
-    const int nc = a.g.ncomp;
-    if (!fast_pointing<C, P, false>(a.g, a.ft, a.fc, qb, qd, nc, T, Pr, pix, w, n, pf))
-        return false;
-    if (n == 0) return true;
-    float *sp = a.signal + det * a.sig_stride + t;
-    float s = *sp;
-#pragma unroll
-    for (int k = 0; k < NT; k++) {
-        if (k >= n) break;
-        long long off, plane;
-        const int bad = locate<P>(a.g, pix[k], &off, &plane);
-        if (bad >= 0) {
-            record_missing_tile(a.err, bad);
-            continue;
-        }
-        if (a.map32) {
-            const float4 m = __ldg(a.map32 + map32_index<P>(a.g, pix[k], off));
-            s = fmaf(m.x, pf[0] * w[k], s);
-            if (nc > 1) s = fmaf(m.y, pf[1] * w[k], s);
-            if (nc > 2) s = fmaf(m.z, pf[2] * w[k], s);
-        } else {
-#pragma unroll
-            for (int c = 0; c < 3; c++)
-                if (c < nc) s = fmaf(d2f_round(__ldg(a.map + off + c * plane)), pf[c] * w[k], s);
-        }
-    }
-    *sp = s;
-    return true;
-}
-
 // Compiled for 5 resident blocks per SM (at most 51 registers; mixed
 // pointing: 7), one variant per pointing mode (0 exact, 1 certified, 2
 // mixed).  The certified and mixed variants of the nearest-neighbour
@@ -143,7 +82,7 @@ __global__ void __launch_bounds__(kBlock, MixedEligible<C, P>::value && MODE == 
     __shared__ int s_queue[!kFastOK ? 1 : (kMixedOK ? 2 : 1) * (kBlock / 32) * kWarpQueue];
     __shared__ WarpPiece s_wp[kFastOK ? kBlock / 32 : 1];
     int det, t0, t1;
-    if (MODE == SO3G_POINTING_CERTIFIED && a.gate.holds()) return;
+    if (MODE != SO3G_POINTING_EXACT && a.gate.holds()) return;
     if (!seg_piece(a.segs, a.piece, det, t0, t1)) return;
     const QuatD ofs = load_quat(a.dets + 4LL * det);
     const float T = __ldg(a.resp + 2 * det), Pr = __ldg(a.resp + 2 * det + 1);
@@ -768,6 +707,14 @@ extern "C" int so3g_proj_from_map(const so3g_pixelization *pz, const double *bor
         }
     }
     L.a.map32 = map32;
+    if (!cert_work) {
+        rc = chunked_bilinear_from_map(pz->coord_sys, kind, L.a, n_det, L.stream, &cert_work);
+        if (rc != 1 && rc != SO3G_OK) {
+            if (map32) cudaFreeAsync(map32, L.stream);
+            bore_f32_free(L.a.bore32, L.stream);
+            return rc;
+        }
+    }
     rc = dispatch_cp(pz->coord_sys, pix_kind(pz), L);
     if (map32) cudaFreeAsync(map32, L.stream);
     bore_f32_free(L.a.bore32, L.stream);

@@ -165,3 +165,37 @@ def test_seam_pole_and_map_edge(gpulib):
     args = [torch.from_numpy(np.ascontiguousarray(x)).cuda()
             for x in (np.asarray(q, dtype=np.float64), dets, resp)]
     _check_all(p.get_ProjEng("TQU"), args, rng)
+
+
+@pytest.mark.parametrize("mode", [_abi.POINTING_MIXED, _abi.POINTING_CERTIFIED])
+@pytest.mark.parametrize("proj,comps", [("ZEA", "TQU"), ("ZEA", "T"), ("TAN", "QU"), ("SIN", "TQU")])
+@pytest.mark.parametrize("n_time,t0,noise", [(3001, 0., 0.), (65, 0., 0.), (4099, 1.7e9, 0.),
+                                             (5000, 0., 1e-8), (5000, 0., 1e-5)])
+def test_bilinear_from_map(gpulib, proj, comps, n_time, t0, noise, mode):
+    """from_map of bilinear zenithal maps: the chunked kernels' weights are
+    the general kernels' or (a coordinate within 2.5e-7 of a pixel of
+    theirs) close to them: 12 products of a map value below |m|, of weights
+    off by at most 2 x 2.5e-7 + 2^-23, and, as nearly all weights are the
+    same floats, within the rounding of a 12-term float32 sum in the mean."""
+    import torch
+    p, args, rng = _inputs("ZEA", 5, n_time, t0=t0, noise=noise)
+    p = synth.car_projectionist((301, 407), synth.ARCMIN, proj=proj, interpol="bilinear")
+    eng = p.get_ProjEng(comps)
+    eng.pointing = mode
+    m = torch.from_numpy(rng.standard_normal((eng.comp_count, 301, 407))).cuda()
+    m[:, ::5, ::7] = 0.
+    sig = torch.from_numpy(rng.standard_normal((5, n_time + 1)).astype(np.float32)).cuda()[:, 1:]
+
+    def scan():
+        out = sig.clone() if n_time % 2 else sig
+        s0 = out.clone()
+        eng.from_map(m, *args, out)
+        d = out.cpu().numpy().copy()
+        out.copy_(s0)
+        return d
+
+    a, b = _both(scan)
+    assert (b != sig.cpu().numpy()).mean() > 0.05
+    d = np.abs(a.astype(np.float64) - b)
+    assert d.max() <= 12 * float(m.abs().max()) * 6.2e-7 + 12 * 2.0**-24 * np.abs(b).max()
+    assert np.sqrt((d**2).mean()) <= np.sqrt(12) * 2.0**-24 * np.sqrt((b.astype(float)**2).mean())
