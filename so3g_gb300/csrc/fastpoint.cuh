@@ -58,6 +58,10 @@ constexpr float kEpsPix = 1e-7f;        // pixel coordinate units
 // within 2.3e-13; P v^2 / D is then within 1.1e-12 max(1, 1/(4D)) P, the
 // zenithal P (alpha^2 / n)^2 within 5e-13 / sqrt(n).
 constexpr float kEpsPf = 3e-12f;
+// With the bilinear pixelizors a sample sent to the exact path gets that path's
+// weights, which may be neighbours of the double-float ones: which samples go
+// there shows in the results' last bits, and stays as it was.
+constexpr float kEpsPfBilinear = 1e-11f;
 
 struct dfl {
     float hi, lo;
@@ -463,7 +467,8 @@ __device__ __forceinline__ bool fast_pixels(const DGeom &g, dfl x, dfl y, int (*
 // accepted.
 template <bool CERT = true>
 __device__ __forceinline__ bool fast_spin(int nc, float T, float Pr, const dfl &Nc,
-                                          const dfl &Ns, const dfl &D, float *pf) {
+                                          const dfl &Ns, const dfl &D, float *pf,
+                                          float eps = kEpsPf) {
     if (nc == 1) {
         pf[0] = T;
         pf[1] = pf[2] = 0.f;
@@ -477,7 +482,7 @@ __device__ __forceinline__ bool fast_spin(int nc, float T, float Pr, const dfl &
     // midpoint to a neighbour, i.e. unless |v.lo| + eps reaches half the
     // gap to the nearer neighbour.
     if (CERT) {
-        const float e = kEpsPf * fmaxf(1.f, 0.25f / D.hi) * fmaxf(1.f, fabsf(Pr));
+        const float e = eps * fmaxf(1.f, 0.25f / D.hi) * fmaxf(1.f, fabsf(Pr));
         if (!(fabsf(v1.hi) > 1e-30f && fabsf(v1.lo) + e < half_gap(v1.hi))) return false;
         if (!(fabsf(v2.hi) > 1e-30f && fabsf(v2.lo) + e < half_gap(v2.hi))) return false;
     }
@@ -664,7 +669,8 @@ __device__ __forceinline__ bool fast_pointing(const DGeom &g, const FastTables &
     const dfl y = df_add(df_mul(Y, fc.inv_cdy), fc.off_y);
     if (!fast_pixels<P>(g, x, y, pix, w, n)) return false;
     if (n == 0) return true;   // off the map: nothing to add
-    return fast_spin<SPIN_CERT>(nc, T, Pr, Nc, Ns, D, pf);
+    return fast_spin<SPIN_CERT>(nc, T, Pr, Nc, Ns, D, pf,
+                                P == PX_FLAT_NT_BL || P == PX_FLAT_T_BL ? kEpsPfBilinear : kEpsPf);
 }
 
 // The rounding step of fast_accum from m's double-float split md.

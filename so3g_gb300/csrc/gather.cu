@@ -395,9 +395,9 @@ struct GatherMxFix {
 // Samples it cannot certify keep their value (the fallback passes add
 // theirs) and are marked in the mask.
 template <int P, int NC>
-__global__ void __launch_bounds__(kBlock, kIxBlocksPerSM)
-    k_from_map_ix4(GatherArgs a, MxMask mm, const IxBore *ixb) {
-    __shared__ IxParams sp[kBlock / 32][32];
+__global__ void __launch_bounds__(kIxBlock, kIxGatherBlocks)
+    k_from_map_ix4(const __grid_constant__ GatherArgs a, MxMask mm, const IxBore *ixb) {
+    __shared__ IxParams sp[kIxWarps][32];
     int det, t0, t1;
     if (!seg_piece(a.segs, a.piece, det, t0, t1)) return;
     const QuatD ofs = load_quat(a.dets + 4LL * det);
@@ -411,12 +411,13 @@ __global__ void __launch_bounds__(kBlock, kIxBlocksPerSM)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tsh = P == PX_HP_T ? __ffsll(a.g.nppt) - 1 : 0;
     const int j0 = t0 / kIxLen, j1 = (t1 - 1) / kIxLen + 1;
-    for (int g = j0 + warp * 32; g < j1; g += (kBlock / 32) * 32) {
-        if (g + lane < j1)
+    const int step = ix_step(j1 - j0);
+    for (int g = j0 + warp * step; g < j1; g += kIxWarps * step) {
+        const int nch = min(step, j1 - g);
+        if (lane < nch)
             ix_setup<P == PX_HP_NT || P == PX_HP_T>(a, ixb, g + lane, a.segs.n_time, qd, q32,
                                                     sp[warp][lane]);
         __syncwarp();
-        const int nch = min(32, j1 - g);
         const int rounds = (nch + 1) / 2;
         for (int r = 0; r < rounds; r++) {
             const int ck = 2 * r + (lane >> 4);
@@ -572,11 +573,11 @@ int gather_interp(const GatherArgs &a, dim3 grid, cudaStream_t stream) {
             return 1;
         }
         if (a.g.ncomp == 1)
-            k_from_map_ix4<P, 1><<<grid, kBlock, 0, stream>>>(a, mm, ixb);
+            k_from_map_ix4<P, 1><<<grid, kIxBlock, 0, stream>>>(a, mm, ixb);
         else if (a.g.ncomp == 2)
-            k_from_map_ix4<P, 2><<<grid, kBlock, 0, stream>>>(a, mm, ixb);
+            k_from_map_ix4<P, 2><<<grid, kIxBlock, 0, stream>>>(a, mm, ixb);
         else
-            k_from_map_ix4<P, 3><<<grid, kBlock, 0, stream>>>(a, mm, ixb);
+            k_from_map_ix4<P, 3><<<grid, kIxBlock, 0, stream>>>(a, mm, ixb);
         int rc = after_launch("from_map (chunked)");
         if (rc == SO3G_OK)
             rc = fix_tiers<0>(GatherIxFix<P>{a, mm}, mm, stream, "from_map (chunked fallback)");

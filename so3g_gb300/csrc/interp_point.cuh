@@ -50,7 +50,20 @@ namespace so3g {
 namespace {
 
 constexpr int kIxLen = 64;            // samples per chunk
-constexpr int kIxBlocksPerSM = 4;
+// Threads per block (its warps are independent) and resident blocks per SM of
+// the chunked kernels.
+constexpr int kIxBlock = 128;
+constexpr int kIxWarps = kIxBlock / 32;
+constexpr int kIxScatterBlocks = 8;
+constexpr int kIxGatherBlocks = 8;
+
+// Chunks of a warp's group for a block that has n: even shares for its warps,
+// in equal groups of at most 32, an even number (a round takes two).
+__device__ __forceinline__ int ix_step(int n) {
+    const int share = (n + kIxWarps - 1) / kIxWarps;
+    const int groups = (share + 31) / 32;
+    return ((share + groups - 1) / groups + 1) & ~1;
+}
 
 // The boresight model of one chunk.
 struct IxBore {
@@ -86,49 +99,52 @@ struct __align__(16) IxParamsHp {
 };
 static_assert(sizeof(IxParamsHp) == sizeof(IxParams), "one shared-memory slot for both");
 
-// The chunks' boresight models (one thread per chunk), in float64.
-__global__ void k_ix_bore(const double *bore, int n_time, int n_chunks, IxBore *out) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n_chunks) return;
+// The chunks' boresight models in float64, 16 threads per chunk (one per
+// quaternion component and quarter of its samples; one thread per chunk, with a
+// root per sample, took 0.14 ms per 500k samples).
+__global__ void __launch_bounds__(128) k_ix_bore(const double *bore, int n_time, int n_chunks,
+                                                 IxBore *out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int chunk = i >> 4, j = min(chunk, n_chunks - 1), comp = i & 3, part = (i >> 2) & 3;
     const int ta = j * kIxLen, tb = min(ta + kIxLen, n_time - 1), L = tb - ta;
-    double qa[4], d1[4], d2[4];
-    for (int k = 0; k < 4; k++) qa[k] = __ldg(bore + 4LL * ta + k);
+    const double *b = bore + 4LL * ta + comp;
+    const double qa = __ldg(b);
+    double d1 = 0., d2 = 0.;
     if (L >= 2) {
-        const int tm = ta + L / 2;
-        const double sm = (double)(tm - ta) / L;
-        for (int k = 0; k < 4; k++) {
-            const double qm = __ldg(bore + 4LL * tm + k), qb = __ldg(bore + 4LL * tb + k);
-            d2[k] = ((qm - qa[k]) - sm * (qb - qa[k])) / (sm * sm - sm);
-            d1[k] = (qb - qa[k]) - d2[k];
-        }
-    } else {
-        for (int k = 0; k < 4; k++) {
-            d1[k] = L == 1 ? __ldg(bore + 4LL * tb + k) - qa[k] : 0.;
-            d2[k] = 0.;
-        }
+        const double sm = (double)(L / 2) / L;
+        const double qm = __ldg(b + 4LL * (L / 2)), qb = __ldg(b + 4LL * L);
+        d2 = ((qm - qa) - sm * (qb - qa)) / (sm * sm - sm);
+        d1 = (qb - qa) - d2;
+    } else if (L == 1) {
+        d1 = __ldg(b + 4) - qa;
     }
-    float f1[4], f2[4];
-    for (int k = 0; k < 4; k++) {
-        f1[k] = __double2float_rn(d1[k]);
-        f2[k] = __double2float_rn(d2[k]);
-    }
-    double e = 0.;
-    for (int t = ta; t <= tb; t++) {
-        const double s = L > 0 ? (double)(t - ta) / L : 0.;
+    const float f1 = __double2float_rn(d1), f2 = __double2float_rn(d2);
+    const double g1 = (double)f1, g2 = (double)f2;
+    double e2 = 0.;
+    bool bad = false;   // NaN (fmax drops it): the chunk is not modelled
+    const int lane0 = threadIdx.x & 28;
+    // 65 samples at most: 17 per part, the last ones clipped to tb.
+    for (int n = 0; n < kIxLen / 4 + 1; n++) {
+        const int k = min(part * (kIxLen / 4) + n, L);
+        const double s = L == kIxLen ? (double)k * (1. / kIxLen) : (L > 0 ? (double)k / L : 0.);
+        const double r = __ldg(b + 4LL * k) - (qa + s * g1 + s * s * g2);
+        const double rr = r * r;
         double n2 = 0.;
-        for (int k = 0; k < 4; k++) {
-            const double r = __ldg(bore + 4LL * t + k) - (qa[k] + s * (double)f1[k] +
-                                                          s * s * (double)f2[k]);
-            n2 += r * r;
-        }
-        e = fmax(e, sqrt(n2));
+#pragma unroll
+        for (int c = 0; c < 4; c++) n2 += __shfl_sync(kFull, rr, lane0 + c);
+        bad |= !(n2 < 1e100);
+        e2 = fmax(e2, n2);
     }
-    IxBore o;
-    o.d1 = make_float4(f1[0], f1[1], f1[2], f1[3]);
-    o.d2 = make_float4(f2[0], f2[1], f2[2], f2[3]);
-    o.e = __double2float_ru(e * (1. + 1e-6) + 1e-30);
-    o.pad[0] = o.pad[1] = o.pad[2] = 0.f;
-    out[j] = o;
+    e2 = fmax(e2, __shfl_xor_sync(kFull, e2, 4));
+    e2 = fmax(e2, __shfl_xor_sync(kFull, e2, 8));
+    bad = __any_sync(kFull, bad);   // (the warp's other chunk as well)
+    if (chunk < n_chunks && part == 0) {
+        float *o = reinterpret_cast<float *>(out + j);
+        o[comp] = f1;
+        o[4 + comp] = f2;
+        if (comp == 0)
+            out[j].e = bad ? 1.f : __double2float_ru(sqrt(e2) * (1. + 1e-6) + 1e-30);
+    }
 }
 
 __device__ __forceinline__ void qmul32(const float (&p)[4], const float (&q)[4], float (&r)[4]) {
@@ -442,14 +458,14 @@ __device__ __forceinline__ bool ix_eval(const IxParams &p, float s, const DGeom 
     const float x = fmaf(s, fmaf(s, fmaf(s, P1.x, P0.w), P0.z), P0.x);
     const float y = fmaf(s, fmaf(s, fmaf(s, P1.w, P1.z), P1.y), P0.y);
     const float fxl = floorf(x), fyl = floorf(y);
-    const bool ok = fabsf((x - fxl) - 0.5f) < P3.z && fabsf((y - fyl) - 0.5f) < P3.w;
+    const bool ok = (fabsf((x - fxl) - 0.5f) < P3.z) & (fabsf((y - fyl) - 0.5f) < P3.w);
     int ix = __float_as_int(P5.x) + (int)fxl, iy = __float_as_int(P5.y) + (int)fyl;
     if constexpr (P == PX_FLAT_T_NN) {
-        on = (unsigned)(ix + 1) < (unsigned)(g.nx + 1) && (unsigned)(iy + 1) < (unsigned)(g.ny + 1);
+        on = ((unsigned)(ix + 1) < (unsigned)(g.nx + 1)) & ((unsigned)(iy + 1) < (unsigned)(g.ny + 1));
         ix = max(ix, 0);
         iy = max(iy, 0);
     } else {
-        on = (unsigned)ix < (unsigned)g.nx && (unsigned)iy < (unsigned)g.ny;
+        on = ((unsigned)ix < (unsigned)g.nx) & ((unsigned)iy < (unsigned)g.ny);
     }
     key = iy * g.nx + ix;
     if constexpr (NC == 1) {
@@ -542,7 +558,8 @@ inline IxBore *ix_bore_models(const double *bore, int n_time, cudaStream_t strea
         cudaGetLastError();
         return nullptr;
     }
-    k_ix_bore<<<(n_chunks + 127) / 128, 128, 0, stream>>>(bore, n_time, n_chunks, p);
+    k_ix_bore<<<(unsigned)((16LL * n_chunks + 127) / 128), 128, 0, stream>>>(bore, n_time, n_chunks,
+                                                                             p);
     if (after_launch("boresight chunk models") != SO3G_OK) {
         cudaFreeAsync(p, stream);
         clear_error();

@@ -248,22 +248,62 @@ __device__ __forceinline__ void ix_flush_run(const ScatterArgs &a, int key, int 
     }
 }
 
+// Runs a warp holds back until there are 32 to flush together (as CxRuns,
+// with one float32 total per value).
+template <int NV>
+struct IxRuns {
+    static constexpr int more = 64;   // most runs a round may add
+    static constexpr int W = (1 + NV + 3) / 4;
+    float4 rec[W][more + 32];
+};
+
+template <int NV>
+__device__ __forceinline__ void ix_run_put(IxRuns<NV> &rb, int pos, int key, const float (&v)[NV]) {
+    constexpr int W = IxRuns<NV>::W;
+    float x[4 * W];
+#pragma unroll
+    for (int k = 0; k < 4 * W; k++)
+        x[k] = k == 0 ? __int_as_float(key) : (k <= NV ? v[k <= NV && k > 0 ? k - 1 : 0] : 0.f);
+#pragma unroll
+    for (int w = 0; w < W; w++)
+        rb.rec[w][pos] = make_float4(x[4 * w], x[4 * w + 1], x[4 * w + 2], x[4 * w + 3]);
+}
+
+// Flushes the last min(32, n) runs held back, one per lane.
+template <int P, bool WEIGHT, int NC, int NV>
+__device__ __forceinline__ void ix_run_flush(const ScatterArgs &a, IxRuns<NV> &rb, int n, int aux,
+                                             const int (&off)[NV]) {
+    constexpr int W = IxRuns<NV>::W;
+    const int i = n - 1 - (int)(threadIdx.x & 31);
+    if (i < 0) return;
+    float x[4 * W], v[NV];
+#pragma unroll
+    for (int w = 0; w < W; w++) {
+        const float4 q = rb.rec[w][i];
+        x[4 * w] = q.x;
+        x[4 * w + 1] = q.y;
+        x[4 * w + 2] = q.z;
+        x[4 * w + 3] = q.w;
+    }
+#pragma unroll
+    for (int k = 0; k < NV; k++) v[k] = x[1 + k];
+    ix_flush_run<P, WEIGHT, NC, NV>(a, __float_as_int(x[0]), aux, off, v);
+}
+
 // to_map / to_weight_map of the chunked pass with four consecutive samples
 // per lane: round r of a group covers its chunks 2r (lanes 0-15) and 2r + 1
 // (lanes 16-31), one float4 of signal per lane (to_map).  A lane sums the
 // runs of equal pixels among its four samples (right to left, at most four
 // float32 terms: each total within 3u of the exact sum of its terms'
-// magnitudes) and packs them into run slots 0..3; slot j of every lane is
-// flushed with one float64 atomic per component in one pass, taken only
-// when some lane has more than j runs.  Runs are a few samples long, so a
-// round of 128 samples takes about two passes of atomics instead of the
-// four that one sample per lane needs, and a fraction of the L2 atomics.
+// magnitudes); its first run is flushed at once with one float64 atomic per
+// component, the others are held back (IxRuns) and flushed 32 at a time.
 // Samples it cannot certify are marked in the mask (bit b of word w = lane
 // 8w + b/4, sample b % 4).
 template <int P, bool WEIGHT, int NC>
-__global__ void __launch_bounds__(kBlock, kIxBlocksPerSM)
-    k_scatter_ix4(ScatterArgs a, MxMask mm, const IxBore *ixb) {
-    __shared__ IxParams sp[kBlock / 32][32];
+__global__ void __launch_bounds__(kIxBlock, kIxScatterBlocks)
+    k_scatter_ix4(const __grid_constant__ ScatterArgs a, MxMask mm, const IxBore *ixb) {
+    __shared__ IxParams sp[kIxWarps][32];
+    __shared__ IxRuns<IxValues<WEIGHT, NC>::NV> s_runs[kIxWarps];
     int det, t0, t1;
     if (!seg_piece(a.segs, a.piece, det, t0, t1)) return;
     float det_wt = 1.f;
@@ -302,12 +342,14 @@ __global__ void __launch_bounds__(kBlock, kIxBlocksPerSM)
         }
         return r;
     };
-    for (int g = j0 + warp * 32; g < j1; g += (kBlock / 32) * 32) {
-        if (g + lane < j1)
+    int nr = 0;   // runs held back
+    const int step = ix_step(j1 - j0);
+    for (int g = j0 + warp * step; g < j1; g += kIxWarps * step) {
+        const int nch = min(step, j1 - g);
+        if (lane < nch)
             ix_setup<P == PX_HP_NT || P == PX_HP_T>(a, ixb, g + lane, a.segs.n_time, qd, q32,
                                                     sp[warp][lane]);
         __syncwarp();
-        const int nch = min(32, j1 - g);
         const int rounds = (nch + 1) / 2;
         const int half = lane >> 4;
         float4 sn = half < nch ? load4((g + half) * kIxLen + (lane & 15) * 4)
@@ -325,15 +367,22 @@ __global__ void __launch_bounds__(kBlock, kIxBlocksPerSM)
             unsigned f4 = 0u;
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const int t = tq + i;
-                const bool live = lane_live && t < t1;
                 int kk = 0;
                 bool on = false;
                 float pf[3];
                 const bool ok = ix_sample<P, NC>(pp, ix_s(pp, tq, i), a.g, T, Pr, kk, on, pf);
-                if (live && !ok) f4 |= 1u << i;
-                key[i] = (live && ok && on) ? kk : -1;
+                if (!ok) f4 |= 1u << i;
+                key[i] = (ok & on) ? kk : -1;
                 V::values(sg[i], pf, det_wt, v[i]);
+            }
+            // A round at the piece's end, or the group's odd last chunk.
+            if ((g + 2 * r + 2) * kIxLen > t1 || 2 * r + 2 > nch) {
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (!(lane_live && tq + i < t1)) {
+                        f4 &= ~(1u << i);
+                        key[i] = -1;
+                    }
             }
             if (__any_sync(kFull, f4 != 0u)) {
                 unsigned x = f4 << (4 * (lane & 7));
@@ -343,43 +392,67 @@ __global__ void __launch_bounds__(kBlock, kIxBlocksPerSM)
                 if ((lane & 7) == 0 && x)
                     mwb[((g + 2 * r) * kIxLen - t0) / 32 + (lane >> 3)] = x;
             }
+            const bool h1 = key[1] != key[0], h2 = key[2] != key[1], h3 = key[3] != key[2];
+            const bool p1 = h1 & (key[1] >= 0), p2 = h2 & (key[2] >= 0), p3 = h3 & (key[3] >= 0);
+            const int n = (int)p1 + (int)p2 + (int)p3;
+            const unsigned c0 = __ballot_sync(kFull, n & 1), c1 = __ballot_sync(kFull, n & 2);
+            const int total = __popc(c0) + 2 * __popc(c1);
             if (a.accum != SO3G_ACCUM_WARP_RUNS) {
+#pragma unroll 1
+                for (int i = 0; i < 4; i++) {
+                    float x[NV];
 #pragma unroll
-                for (int i = 0; i < 4; i++)
-                    ix_flush_run<P, WEIGHT, NC, NV>(a, key[i], aux, off, v[i]);
+                    for (int k = 0; k < NV; k++)
+                        x[k] = i == 0 ? v[0][k] : (i == 1 ? v[1][k] : (i == 2 ? v[2][k] : v[3][k]));
+                    ix_flush_run<P, WEIGHT, NC, NV>(
+                        a, i == 0 ? key[0] : (i == 1 ? key[1] : (i == 2 ? key[2] : key[3])), aux,
+                        off, x);
+                }
                 continue;
             }
-            // Run heads and right-to-left run totals (in place: v[i] becomes
-            // the total of the run from i while i is in it).
-            const bool h1 = key[1] != key[0], h2 = key[2] != key[1], h3 = key[3] != key[2];
+            // Right-to-left run totals (in place: v[i] becomes the total of
+            // the run from i while i is in it).
 #pragma unroll
             for (int k = 0; k < NV; k++) {
                 if (!h3) v[2][k] += v[3][k];
                 if (!h2) v[1][k] += v[2][k];
                 if (!h1) v[0][k] += v[1][k];
             }
-            // Slots 1 and 2: the first and second heads among samples 1..3;
-            // slot 3: sample 3 when all three are heads.
-            const int nruns = 1 + h1 + h2 + h3;
-            int ks1 = key[3], ks2 = key[3];
-            float s1[NV], s2[NV];
-#pragma unroll
-            for (int k = 0; k < NV; k++) {
-                s1[k] = h1 ? v[1][k] : (h2 ? v[2][k] : v[3][k]);
-                s2[k] = (h1 && h2) ? v[2][k] : v[3][k];
-            }
-            ks1 = h1 ? key[1] : (h2 ? key[2] : key[3]);
-            ks2 = (h1 && h2) ? key[2] : key[3];
             ix_flush_run<P, WEIGHT, NC, NV>(a, key[0], aux, off, v[0]);
-            if (__any_sync(kFull, nruns > 1) && nruns > 1)
-                ix_flush_run<P, WEIGHT, NC, NV>(a, ks1, aux, off, s1);
-            if (__any_sync(kFull, nruns > 2) && nruns > 2)
-                ix_flush_run<P, WEIGHT, NC, NV>(a, ks2, aux, off, s2);
-            if (__any_sync(kFull, nruns > 3) && nruns > 3)
-                ix_flush_run<P, WEIGHT, NC, NV>(a, key[3], aux, off, v[3]);
+            // The further runs: held back, unless there are too many.
+            const unsigned lt = (1u << lane) - 1u;
+            if (total <= IxRuns<NV>::more) {
+                int pos = nr + __popc(c0 & lt) + 2 * __popc(c1 & lt);
+                if (p1) ix_run_put<NV>(s_runs[warp], pos, key[1], v[1]);
+                pos += p1;
+                if (p2) ix_run_put<NV>(s_runs[warp], pos, key[2], v[2]);
+                pos += p2;
+                if (p3) ix_run_put<NV>(s_runs[warp], pos, key[3], v[3]);
+                nr += total;
+            } else {
+                // Nearly every sample is a run of its own: no buffer needed.
+#pragma unroll 1
+                for (int i = 1; i < 4; i++) {
+                    float x[NV];
+#pragma unroll
+                    for (int k = 0; k < NV; k++)
+                        x[k] = i == 1 ? v[1][k] : (i == 2 ? v[2][k] : v[3][k]);
+                    const bool head = i == 1 ? p1 : (i == 2 ? p2 : p3);
+                    if (head)
+                        ix_flush_run<P, WEIGHT, NC, NV>(
+                            a, i == 1 ? key[1] : (i == 2 ? key[2] : key[3]), aux, off, x);
+                }
+            }
+            __syncwarp();
+            while (nr >= 32) {
+                ix_run_flush<P, WEIGHT, NC, NV>(a, s_runs[warp], nr, aux, off);
+                nr -= 32;
+                __syncwarp();
+            }
         }
         __syncwarp();
     }
+    if (nr > 0) ix_run_flush<P, WEIGHT, NC, NV>(a, s_runs[warp], nr, aux, off);
 }
 
 // The fallback passes of k_scatter_ix4, by tier: 0 the float32 tier, 1 the
@@ -479,11 +552,11 @@ int scatter_interp(const ScatterArgs &a, dim3 grid, cudaStream_t stream) {
             return 1;
         }
         if (nc == 1)
-            k_scatter_ix4<P, WEIGHT, 1><<<grid, kBlock, 0, stream>>>(a, mm, ixb);
+            k_scatter_ix4<P, WEIGHT, 1><<<grid, kIxBlock, 0, stream>>>(a, mm, ixb);
         else if (nc == 2)
-            k_scatter_ix4<P, WEIGHT, 2><<<grid, kBlock, 0, stream>>>(a, mm, ixb);
+            k_scatter_ix4<P, WEIGHT, 2><<<grid, kIxBlock, 0, stream>>>(a, mm, ixb);
         else
-            k_scatter_ix4<P, WEIGHT, 3><<<grid, kBlock, 0, stream>>>(a, mm, ixb);
+            k_scatter_ix4<P, WEIGHT, 3><<<grid, kIxBlock, 0, stream>>>(a, mm, ixb);
         int rc = after_launch(WEIGHT ? "to_weight_map (chunked)" : "to_map (chunked)");
         if (rc == SO3G_OK)
             rc = fix_tiers<0>(ScatterIxFix<P, WEIGHT>{a, mm}, mm, stream,
