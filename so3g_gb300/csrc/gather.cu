@@ -554,11 +554,16 @@ struct GatherIxFix {
 // and for HEALPix maps (tiled maps: the float32 copy spans the parent map);
 // returns 1 (nothing launched) where it does not apply.
 template <int C, int P>
-int gather_interp(const GatherArgs &a, dim3 grid, cudaStream_t stream) {
+int gather_interp(const GatherArgs &args, dim3 grid, cudaStream_t stream) {
     if constexpr (!(C == SO3G_COORD_CAR && (P == PX_FLAT_NT_NN || P == PX_FLAT_T_NN ||
                                             P == PX_HP_NT || P == PX_HP_T))) {
         return 1;
     } else {
+        GatherArgs a = args;
+        if (!a.segs.seg) {
+            a.piece = ix_piece(a.piece, a.segs.n_time);
+            grid.y = (unsigned)((a.segs.n_time + (long long)a.piece - 1) / a.piece);
+        }
         const long long npix =
             (P == PX_FLAT_NT_NN || P == PX_FLAT_T_NN) ? (long long)a.g.ny * a.g.nx : a.g.npix;
         if (a.segs.seg || a.segs.n_time < 2 || !a.map32 || npix >= (1LL << 31) ||

@@ -51,11 +51,20 @@ namespace {
 
 constexpr int kIxLen = 64;            // samples per chunk
 // Threads per block (its warps are independent) and resident blocks per SM of
-// the chunked kernels.
+// the chunked kernels, and the longest piece: a full group for each warp.
 constexpr int kIxBlock = 128;
 constexpr int kIxWarps = kIxBlock / 32;
 constexpr int kIxScatterBlocks = 8;
 constexpr int kIxGatherBlocks = 8;
+constexpr int kIxPiece = 2 * kIxWarps * 32 * kIxLen;
+
+// Pieces of the chunked kernels: as the call's, at most kIxPiece long (as far
+// as the grid's limit allows).
+inline int ix_piece(int piece, long long n_time) {
+    long long p = piece < kIxPiece ? piece : kIxPiece;
+    while ((n_time + p - 1) / p > 65535) p *= 2;
+    return (int)p;
+}
 
 // Chunks of a warp's group for a block that has n: even shares for its warps,
 // in equal groups of at most 32, an even number (a round takes two).
@@ -126,12 +135,22 @@ __global__ void __launch_bounds__(128) k_ix_bore(const double *bore, int n_time,
     // 65 samples at most: 17 per part, the last ones clipped to tb.
     for (int n = 0; n < kIxLen / 4 + 1; n++) {
         const int k = min(part * (kIxLen / 4) + n, L);
-        const double s = L == kIxLen ? (double)k * (1. / kIxLen) : (L > 0 ? (double)k / L : 0.);
-        const double r = __ldg(b + 4LL * k) - (qa + s * g1 + s * s * g2);
+        // s = k / L and s^2; both exact floats for a whole chunk, and then
+        // converted without the float64 pipe.
+        double s, ss;
+        if (L == kIxLen) {
+            const float sf = (float)k * (1.f / kIxLen);
+            s = f2d(sf);
+            ss = f2d(sf * sf);
+        } else {
+            s = L > 0 ? (double)k / L : 0.;
+            ss = s * s;
+        }
+        const double r = __ldg(b + 4LL * k) - (qa + s * g1 + ss * g2);
         const double rr = r * r;
-        double n2 = 0.;
+        double n2 = __shfl_sync(kFull, rr, lane0);
 #pragma unroll
-        for (int c = 0; c < 4; c++) n2 += __shfl_sync(kFull, rr, lane0 + c);
+        for (int c = 1; c < 4; c++) n2 += __shfl_sync(kFull, rr, lane0 + c);
         bad |= !(n2 < 1e100);
         e2 = fmax(e2, n2);
     }

@@ -530,11 +530,16 @@ struct ScatterMxFix {
 // (no sample segments); returns 1 (nothing launched) where it does not
 // apply or an allocation fails.
 template <int C, int P, bool WEIGHT>
-int scatter_interp(const ScatterArgs &a, dim3 grid, cudaStream_t stream) {
+int scatter_interp(const ScatterArgs &args, dim3 grid, cudaStream_t stream) {
     if constexpr (!(C == SO3G_COORD_CAR && (P == PX_FLAT_NT_NN || P == PX_FLAT_T_NN ||
                                             P == PX_HP_NT || P == PX_HP_T))) {
         return 1;
     } else {
+        ScatterArgs a = args;
+        if (!a.segs.seg) {
+            a.piece = ix_piece(a.piece, a.segs.n_time);
+            grid.y = (unsigned)((a.segs.n_time + (long long)a.piece - 1) / a.piece);
+        }
         // Keys and plane offsets (key + plane offset untiled; within a tile
         // tiled) in 32 bits.
         const long long nc = a.g.ncomp;
