@@ -29,7 +29,7 @@ UNITS = ["api.cu", "pointing.cu", "scatter.cu", "scatter_weight.cu", "gather.cu"
 HEADERS = ["device.cuh", "host.h", "scatter_kernel.cuh", "scatter_launch.cuh", "batch_launch.cuh",
            "fastpoint.cuh", "mixedpoint.cuh", "mixed_launch.cuh", "mx_common.cuh", "interp_point.cuh",
            "cert_point.cuh", "cert_scatter.cuh", "gather_kernel.cuh",
-           "cert_map.cuh"]
+           "cert_map.cuh", "pair32.cuh"]
 
 
 def nvcc():

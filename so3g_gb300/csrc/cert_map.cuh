@@ -3,6 +3,7 @@
 #pragma once
 
 #include "host.h"
+#include "pair32.cuh"
 
 namespace so3g {
 
@@ -83,6 +84,49 @@ __device__ __forceinline__ bool cx_accum(float &sig, float h, float l, float pf)
         ok = true;
     }
     if (ok) sig = r;
+    return ok;
+}
+
+// The same for one component of two samples, without the exact zeros: c0 and
+// c1 become false where a rounding is not certain (or the sum is zero).
+__device__ __forceinline__ void cx_accum2(float &s0, float &s1, float h0, float h1, float l0,
+                                          float l1, float f0, float f1, bool &c0, bool &c1) {
+    const float p0 = h0 * f0, p1 = h1 * f1;
+    const f32x2 s = f2_make(s0, s1), p = f2_make(p0, p1);
+    const f32x2 pe = f2_make(fmaf(l0, f0, fmaf(h0, f0, -p0)), fmaf(l1, f1, fmaf(h1, f1, -p1)));
+    f32x2 S, x;
+    f2_two_sum(s, p, S, x);
+    const f32x2 L = f2_add(x, pe);
+    const f32x2 e = f2_mul(f2_both(5e-13f),
+                           f2_make(fabsf(p0) + fabsf(s0), fabsf(p1) + fabsf(s1)));
+    float q0, q1;
+    f2_get(f2_add(S, f2_add(L, e)), s0, s1);
+    f2_get(f2_add(S, f2_sub(L, e)), q0, q1);
+    c0 = c0 & (s0 == q0) & (fabsf(s0) > 1e-30f);
+    c1 = c1 & (s1 == q1) & (fabsf(s1) > 1e-30f);
+}
+
+// All NC components of one sample, one after the other (a sample that
+// cx_accum2 did not take); out: the sum.
+template <int NC, int W>
+__device__ __noinline__ bool cx_accum_slow(float sig, float4 m0, float4 m1, float f0, float f1,
+                                           float f2, float *out) {
+    const float hl[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w}, pf[3] = {f0, f1, f2};
+    bool ok = true;
+#pragma unroll
+    for (int c = 0; c < NC; c++) ok = ok & cx_accum(sig, hl[2 * c], hl[2 * c + 1], pf[c]);
+    *out = sig;
+    return ok;
+}
+template <int NC, int W>
+__device__ __forceinline__ bool cx_accum_all(float sig, const float (&hl)[4 * W],
+                                             const float (&pf)[3], float &out) {
+    const float4 m0 = make_float4(hl[0], hl[1], hl[2], hl[3]);
+    const float4 m1 = W > 1 ? make_float4(hl[4 * W - 4], hl[4 * W - 3], hl[4 * W - 2], hl[4 * W - 1])
+                            : make_float4(0.f, 0.f, 0.f, 0.f);
+    float r;
+    const bool ok = cx_accum_slow<NC, W>(sig, m0, m1, pf[0], pf[1], pf[2], &r);
+    out = r;
     return ok;
 }
 

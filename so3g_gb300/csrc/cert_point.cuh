@@ -41,6 +41,7 @@
 #pragma once
 
 #include "host.h"
+#include "pair32.cuh"
 
 namespace so3g {
 
@@ -80,9 +81,11 @@ struct CxModel {
 
 // Per (detector, chunk), nine 16-byte words (an odd number: neighbouring
 // chunks' slots start on different shared-memory banks):
-//   0: x0 x1 x2 x3   1: y0 y1 y2 y3   2: hx hy e -   3: xb yb mid flag
-//   4: f0 f1 l0 l1   5: a2 a3 a4 g0x  6: f0 f1 l0 l1   7: a2 a3 a4 g0y
-//   8: g0z g1x g1y g1z
+//   0: x0 y0 x1 y1   1: x2 y2 x3 y3   2: hx hy e e   3: xb yb mid flag
+//   4: f0 h0 f1 h1   5: l0 m0 l1 m1   6: a2 b2 a3 b3   7: a4 b4 g1x g1y
+//   8: g0x g0y g0z g1z
+// (two quantities side by side: x and y, the two spin factors, so that one
+// f32x2 instruction takes both).
 // With k = t - mid: x = xb + 1/2 + x0 + k (x1 + k (x2 + k x3)) (xb less the
 // bits of kCxMagic); a spin factor is
 // (f0 + k f1), exact in float32, plus the correction l0 + k (l1 + k (a2 + k
@@ -94,8 +97,8 @@ constexpr int kCxWords = 9;
 // The bilinear form (TAN, ZEA, SIN; thirteen words) holds the pixel
 // coordinates as the spin factors are, exact part plus correction, and their
 // gradients per residual unit:
-//   0: fx0 fx1 lx0 lx1   1: x2 x3 x4 e   2: fy0 fy1 ly0 ly1   3: xb yb mid flag
-//   4 .. 8: as above   9: y2 y3 y4 -   10, 11, 12: jx0 jx1 jy0 jy1 for the
+//   0: fx0 fy0 fx1 fy1   1: x2 y2 x3 y3   2: lx0 ly0 lx1 ly1   3: xb yb mid flag
+//   4 .. 8: as above   9: x4 y4 e e   10, 11, 12: jx0 jy0 jx1 jy1 for the
 //   residual's components x, y, z (each g0 + k g1)
 // with the unmodelled chunks' e = -1 (pixel bound kCxBlPix).
 constexpr int kCxBlWords = 13;
@@ -362,7 +365,7 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
     constexpr bool SPIN = NC > 1;
     constexpr float u = kU;
     const int mid = cx_mid(j, n_time);
-    if (BL) w[1] = make_float4(0.f, 0.f, 0.f, -1.f);
+    if (BL) w[9] = make_float4(0.f, 0.f, -1.f, -1.f);
     w[2] = make_float4(-1.f, -1.f, 0.f, 0.f);
     w[3] = make_float4(0.f, 0.f, __int_as_float(mid), 0.f);
     const CxBore &cb = cxb[j];
@@ -663,10 +666,11 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
                          (lsb > 0.f ? rx * ai * (E * (16.f * E + 2.f * zz + 32.f * u) + 2.f * lsb)
                                     : rx * ai * E);
         if (!(eb < kCxBlPix && (sx * aix + 1.f) < 60.f && (sy * aiy + 1.f) < 60.f)) return;
-        w[0] = make_float4(fx0, fx1, (fx.hi - fx0) + fx.lo, (vx.hi - fx1) + vx.lo);
-        w[1] = make_float4(x2, x3, x4p, -1.f);
-        w[2] = make_float4(fy0, fy1, (fy.hi - fy0) + fy.lo, (vy.hi - fy1) + vy.lo);
-        w[9] = make_float4(y2, y3, y4p, 0.f);
+        w[0] = make_float4(fx0, fy0, fx1, fy1);
+        w[1] = make_float4(x2, y2, x3, y3);
+        w[2] = make_float4((fx.hi - fx0) + fx.lo, (fy.hi - fy0) + fy.lo, (vx.hi - fx1) + vx.lo,
+                           (vy.hi - fy1) + vy.lo);
+        w[9] = make_float4(x4p, y4p, -1.f, -1.f);
         if (lsb > 0.f) {
             float N0[4], N1[4], gx0[3], gx1[3], gy0[3], gy1[3];
 #pragma unroll
@@ -680,12 +684,12 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
             const float dx = lsb * s1 * icx, dy = lsb * s1 * icy;
 #pragma unroll
             for (int c = 0; c < 3; c++)
-                w[10 + c] = make_float4((gx0[c] + gx1[c]) * hx, (gx1[c] - gx0[c]) * dx,
-                                        (gy0[c] + gy1[c]) * hy, (gy1[c] - gy0[c]) * dy);
+                w[10 + c] = make_float4((gx0[c] + gx1[c]) * hx, (gy0[c] + gy1[c]) * hy,
+                                        (gx1[c] - gx0[c]) * dx, (gy1[c] - gy0[c]) * dy);
         }
     } else {
-    w[0] = make_float4(xf, cx1 * icx * s1, cx2 * icx * s2, cx3 * icx * s3);
-    w[1] = make_float4(yf, cy1 * icy * s1, cy2 * icy * s2, cy3 * icy * s3);
+        w[0] = make_float4(xf, yf, cx1 * icx * s1, cy1 * icy * s1);
+        w[1] = make_float4(cx2 * icx * s2, cy2 * icy * s2, cx3 * icx * s3, cy3 * icy * s3);
     }
     float e = 0.f;
     bool flag = BL && lsb > 0.f;
@@ -728,6 +732,7 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         const bool fine = pe > 24 && pe < 250 && fabsf(p1) < 0.5f;
         const float cst = fine ? 3.f * __int_as_float(pe << 23) : 0.f;
         const float gr = fine ? __int_as_float((pe - 22) << 23) : 0.f;
+        float o[2][7];
 #pragma unroll
         for (int f = 0; f < 2; f++) {
             // F1's terms: Re(c_k (F1 + i F2)); F2's: Im.
@@ -738,9 +743,18 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
             const float l0 = (F.hi - f0) + F.lo, l1 = (q1.hi - f1) + q1.lo;
             const float a2 = fmaf(phi2, G.hi, df_mul(hp2, F).hi);
             const float a3 = c3.r * F.hi + c3.i * G.hi, a4 = c4.r * F.hi + c4.i * G.hi;
-            w[4 + 2 * f] = make_float4(f0, f1, l0, l1);
-            w[5 + 2 * f] = make_float4(a2 * s2, a3 * s3, a4 * s4, 0.f);
+            o[f][0] = f0;
+            o[f][1] = f1;
+            o[f][2] = l0;
+            o[f][3] = l1;
+            o[f][4] = a2 * s2;
+            o[f][5] = a3 * s3;
+            o[f][6] = a4 * s4;
         }
+        w[4] = make_float4(o[0][0], o[1][0], o[0][1], o[1][1]);
+        w[5] = make_float4(o[0][2], o[1][2], o[0][3], o[1][3]);
+        w[6] = make_float4(o[0][4], o[1][4], o[0][5], o[1][5]);
+        w[7] = make_float4(o[0][6], o[1][6], 0.f, 0.f);
         // e: the double-float error and the reference's roundings (kEpsPf;
         // phi1's is of the same size), the terms left out, a norm off 1
         // (CAR's reference divides by (1 - sin^2) / 4, the model by
@@ -772,26 +786,51 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
             e += aP * (E * (2.1f * gerr + km * (64.f * u + 4.f * eta)) + 16.f * km * km * E * E +
                        2.f * (km + 4.f) * lsb);
             const float hm = 0.5f * lsb, hd = lsb * s1;
-            w[5].w = (g0[0] + g1[0]) * hm;
-            w[7].w = (g0[1] + g1[1]) * hm;
-            w[8] = make_float4((g0[2] + g1[2]) * hm, (g1[0] - g0[0]) * hd, (g1[1] - g0[1]) * hd,
+            w[7].z = (g1[0] - g0[0]) * hd;
+            w[7].w = (g1[1] - g0[1]) * hd;
+            w[8] = make_float4((g0[0] + g1[0]) * hm, (g0[1] + g1[1]) * hm, (g0[2] + g1[2]) * hm,
                                (g1[2] - g0[2]) * hd);
         } else {
             e += aP * (4.3f + 2.2f * rsqrtf(Df)) * E;
         }
         if (!fine) e = __int_as_float(0x7f800000);   // never certain
     }
-    if constexpr (BL) w[1].w = e;
-    else w[2] = make_float4(HP ? ex : 0.5f - ex, HP ? ey : 0.5f - ey, e, 0.f);
+    if constexpr (BL) w[9].z = w[9].w = e;
+    else w[2] = make_float4(HP ? ex : 0.5f - ex, HP ? ey : 0.5f - ey, e, e);
     w[3] = make_float4(__int_as_float(xb), __int_as_float(yb), __int_as_float(mid),
                        flag ? 1.f : 0.f);
 }
 
-// The exact part and the correction of a spin factor at k = t - mid.
-__device__ __forceinline__ void cx_factor(const float4 &A, const float4 &B, float k, float &S,
-                                          float &L) {
-    L = fmaf(k, fmaf(k, fmaf(k, fmaf(k, B.z, B.y), B.x), A.w), A.z);
-    S = fmaf(k, A.y, A.x);
+__device__ __forceinline__ f32x2 cx_lo(const float4 &w) { return f2_make(w.x, w.y); }
+__device__ __forceinline__ f32x2 cx_hi(const float4 &w) { return f2_make(w.z, w.w); }
+
+// The exact parts S and corrections L of the spin factors at k = t - mid
+// (k2: in both halves), with the residual's turn where `flag` is set.
+__device__ __forceinline__ void cx_factors(const float4 *w, f32x2 k2, const float (&res)[3],
+                                           bool flag, f32x2 &S, f32x2 &L) {
+    const float4 W4 = w[4], W5 = w[5], W6 = w[6], W7 = w[7];
+    L = f2_fma(k2, f2_fma(k2, f2_fma(k2, f2_fma(k2, cx_lo(W7), cx_hi(W6)), cx_lo(W6)), cx_hi(W5)),
+               cx_lo(W5));
+    S = f2_fma(k2, cx_hi(W4), cx_lo(W4));
+    if (flag) {
+        const float4 W8 = w[8];
+        float k, k_, gx, gy, S1, S2, L1, L2;
+        f2_get(k2, k, k_);
+        f2_get(f2_fma(k2, cx_hi(W7), cx_lo(W8)), gx, gy);
+        f2_get(S, S1, S2);
+        f2_get(L, L1, L2);
+        const float dphi = fmaf(gx, res[0], fmaf(gy, res[1], fmaf(k, W8.w, W8.z) * res[2]));
+        L = f2_make(fmaf(-S2, dphi, L1), fmaf(S1, dphi, L2));
+    }
+}
+
+// Their float32 values (within e2 of S + L); false when a rounding is not
+// certain.
+__device__ __forceinline__ bool cx_round(f32x2 S, f32x2 L, f32x2 e2, float &v1, float &v2) {
+    float u1, u2;
+    f2_get(f2_add(S, f2_add(L, e2)), v1, v2);
+    f2_get(f2_add(S, f2_sub(L, e2)), u1, u2);
+    return (v1 == u1) & (v2 == u2);
 }
 
 // The HEALPix pixel of longitude x (error ex; < 0: none) and sin(lat) y (ey),
@@ -810,7 +849,7 @@ static __device__ __noinline__ int cx_hp_pixel(int nside, int nest, int npix, fl
     return hp_pixel_f32<P, P == PX_HP_T, true>(g, x, ex, y, ey, 0.f, 0.f, pix) ? pix[0] : -1;
 }
 
-// One sample (k = t - mid) of a modelled chunk: pixel key (flat: iy * nx +
+// One sample (k2: t - mid in both halves) of a modelled chunk: pixel key (flat: iy * nx +
 // ix, of the parent map when tiled; HEALPix: the pixel), on the map or not,
 // and the spin factors of an NC-component map; false when the pixel or
 // (on the map) a spin factor is not certain.  res: the sample's residual
@@ -819,14 +858,16 @@ static __device__ __noinline__ int cx_hp_pixel(int nside, int nest, int npix, fl
 // A spin factor is within e of S + L (S exact), so the reference's value
 // rounds to the same float32 when S + (L + e) and S + (L - e) do.
 template <int P, int NC>
-__device__ __forceinline__ bool cx_sample(const float4 *w, float k, const float (&res)[3],
+__device__ __forceinline__ bool cx_sample(const float4 *w, f32x2 k2, const float (&res)[3],
                                           bool flag, const DGeom &g, float T, int &key, bool &on,
                                           float (&pf)[3]) {
     const float4 P0 = w[0], P1 = w[1], P2 = w[2];
-    const float x = fmaf(k, fmaf(k, fmaf(k, P0.w, P0.z), P0.y), P0.x);
-    const float y = fmaf(k, fmaf(k, fmaf(k, P1.w, P1.z), P1.y), P1.x);
+    const f32x2 xy =
+        f2_fma(k2, f2_fma(k2, f2_fma(k2, cx_hi(P1), cx_lo(P1)), cx_hi(P0)), cx_lo(P0));
     bool ok;
     if constexpr (P == PX_HP_NT || P == PX_HP_T) {
+        float x, y;
+        f2_get(xy, x, y);
         key = cx_hp_pixel<P>((int)g.nside, g.nest, (int)g.npix, x, P2.x, y, P2.y);
         ok = key >= 0;
         on = true;
@@ -834,8 +875,11 @@ __device__ __forceinline__ bool cx_sample(const float4 *w, float k, const float 
         const float4 P3 = w[3];
         // x, y less 1/2: the nearest integer is the floor, and the distance
         // from it the fraction less 1/2.
-        const float rx = x + kCxMagic, ry = y + kCxMagic;
-        ok = (fabsf(x - (rx - kCxMagic)) < P2.x) & (fabsf(y - (ry - kCxMagic)) < P2.y);
+        const f32x2 magic = f2_both(kCxMagic), r2 = f2_add(xy, magic);
+        float rx, ry, dx, dy;
+        f2_get(r2, rx, ry);
+        f2_get(f2_sub(xy, f2_sub(r2, magic)), dx, dy);
+        ok = (fabsf(dx) < P2.x) & (fabsf(dy) < P2.y);
         int ix = __float_as_int(P3.x) + __float_as_int(rx),
             iy = __float_as_int(P3.y) + __float_as_int(ry);
         if constexpr (P == PX_FLAT_T_NN) {
@@ -852,19 +896,10 @@ __device__ __forceinline__ bool cx_sample(const float4 *w, float k, const float 
         pf[0] = T;
         pf[1] = pf[2] = 0.f;
     } else {
-        float S1, L1, S2, L2;
-        const float4 W5 = w[5], W7 = w[7];
-        cx_factor(w[4], W5, k, S1, L1);
-        cx_factor(w[6], W7, k, S2, L2);
-        if (flag) {
-            const float4 W8 = w[8];
-            const float dphi = fmaf(fmaf(k, W8.y, W5.w), res[0],
-                                    fmaf(fmaf(k, W8.z, W7.w), res[1], fmaf(k, W8.w, W8.x) * res[2]));
-            L1 = fmaf(-S2, dphi, L1);
-            L2 = fmaf(S1, dphi, L2);
-        }
-        const float v1 = S1 + (L1 + P2.z), v2 = S2 + (L2 + P2.z);
-        const bool c = (v1 == S1 + (L1 - P2.z)) & (v2 == S2 + (L2 - P2.z));
+        f32x2 S, L;
+        cx_factors(w, k2, res, flag, S, L);
+        float v1, v2;
+        const bool c = cx_round(S, L, cx_hi(P2), v1, v2);
         ok = ok & (c | !on);
         if constexpr (NC == 2) {
             pf[0] = v1;

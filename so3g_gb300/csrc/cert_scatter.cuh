@@ -12,11 +12,12 @@
 // do not certify go to a list and from there through the per-sample
 // certified path and, if need be, the float64 one (k_scatter_cx_fix).
 //
-// Bound by instruction issue (~230 warp-instructions per 32 samples, the
+// Bound by instruction issue (~200 warp-instructions per 32 samples, the
 // per-sample path ~910), then by the L2 atomic units.  CAR TQU 3 x 2000 x
-// 2000, 1000 det x 1M samples: to_map 26.2 -> 8.7 ms (of which 0.9 ms the
-// fallback), to_weight_map of 500 x 500k 7.3 -> 3.3 ms; HEALPix nside 1024,
-// 400 det x 500k, to_map + from_map 15.6 -> 6.5 ms.
+// 2000, 1000 det x 1M samples: to_map 26.2 -> 8.3 ms, with f32x2 instructions
+// for the coordinates, the spin factors and the runs' sums 8.0 ms (of which
+// 1.2 ms the fallback), to_weight_map of 500 x 500k 7.3 -> 2.8 ms; HEALPix
+// nside 1024, 400 det x 500k, to_map + from_map 15.6 -> 5.6 ms.
 #pragma once
 
 #include <algorithm>
@@ -198,6 +199,24 @@ __device__ __forceinline__ void cx_run_flush(const ScatterArgs &a, CxRuns<NV> &r
     cx_flush<P, WEIGHT, NC, NV>(a, __float_as_int(x[0]), aux, plane, hi, lo);
 }
 
+// The total a of a run (a term) plus b's, the roundings in lo.
+template <int NV>
+__device__ __forceinline__ void cx_join(float (&a)[NV], float (&lo)[NV], const float (&b)[NV],
+                                        const float (&blo)[NV]) {
+    if constexpr (NV & 1) {
+        float e;
+        two_sum(a[0], b[0], a[0], e);
+        lo[0] = blo[0] + e;
+    }
+#pragma unroll
+    for (int c = NV & 1; c + 1 < NV; c += 2) {
+        f32x2 s, e;
+        f2_two_sum(f2_make(a[c], a[c + 1]), f2_make(b[c], b[c + 1]), s, e);
+        f2_get(s, a[c], a[c + 1]);
+        f2_get(f2_add(f2_make(blo[c], blo[c + 1]), e), lo[c], lo[c + 1]);
+    }
+}
+
 // The runs of equal pixels among a lane's four samples: the first flushed,
 // the others held back (nr: runs held back so far; flushed down to fewer
 // than 32).  False (nothing done) when the round has too many further
@@ -221,13 +240,9 @@ __device__ __forceinline__ bool cx_runs4(const ScatterArgs &a, CxRuns<NV> &rb, i
             lo[j][c] = 0.f;
         }
     // Right to left: v[i] + lo[i] becomes the total of the run from i on.
-#pragma unroll
-    for (int c = 0; c < NV; c++) {
-        float e;
-        if (!h3) { two_sum(v[2][c], v[3][c], v[2][c], e); lo[2][c] = e; }
-        if (!h2) { two_sum(v[1][c], v[2][c], v[1][c], e); lo[1][c] = lo[2][c] + e; }
-        if (!h1) { two_sum(v[0][c], v[1][c], v[0][c], e); lo[0][c] = lo[1][c] + e; }
-    }
+    if (!h3) cx_join<NV>(v[2], lo[2], v[3], lo[3]);
+    if (!h2) cx_join<NV>(v[1], lo[1], v[2], lo[2]);
+    if (!h1) cx_join<NV>(v[0], lo[0], v[1], lo[1]);
     if (total) {
         const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
         int pos = nr + __popc(b0 & lt) + 2 * __popc(b1 & lt);
@@ -352,8 +367,8 @@ __global__ void __launch_bounds__(kCxBlock, CxScatterBlocks<WEIGHT>::value)
             for (int i = 0; i < 4; i++) {
                 int kk = 0;
                 bool on = false;
-                const bool ok = cx_sample<P, NC>(w, kq + (float)i, res[i], w3.w != 0.f, a.g, T, kk,
-                                                  on, pf[i]);
+                const bool ok = cx_sample<P, NC>(w, f2_both(kq + (float)i), res[i], w3.w != 0.f,
+                                                  a.g, T, kk, on, pf[i]);
                 if (!ok) f4 |= 1u << i;
                 key[i] = (ok & on) ? kk : -1;
             }

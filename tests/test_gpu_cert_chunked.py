@@ -106,6 +106,29 @@ def test_geometries(gpulib, geom, comps):
     _check_all(p.get_ProjEng(comps), args, rng)
 
 
+@pytest.mark.parametrize("comps", ["T", "QU", "TQU"])
+@pytest.mark.parametrize("geom", ["CAR", "CAR-tiled", "HP-NEST"])
+def test_from_map_onto_zeros(gpulib, geom, comps):
+    """Sums that are exact zeros of either sign, subnormal or tiny: a third
+    of the map zero, rows that start from +-0 and at the end of float32's
+    range, a detector without polarisation response."""
+    import torch
+    p, args, rng = _inputs(geom, 6, 3003, el=45.)
+    args[2][2, 1] = 0.0
+    eng = p.get_ProjEng(comps)
+    m = eng.zeros(eng.comp_count, device="cuda")
+    for t in (m if isinstance(m, list) else [m]):
+        x = rng.standard_normal(tuple(t.shape)) * 10. ** rng.integers(-42, 2, tuple(t.shape))
+        x[rng.random(tuple(t.shape)) < 0.2] = 0.0
+        x[rng.random(tuple(t.shape)) < 0.2] = -0.0
+        t.copy_(torch.from_numpy(x))
+    sig = torch.zeros((6, 3003), dtype=torch.float32, device="cuda")
+    sig[1::3] = -0.0
+    sig[5] = 1e-39
+    a, b = (x.cpu().numpy() for x in _both(lambda: eng.from_map(m, *args, sig.clone())))
+    assert (b != 0).any() and bits_equal(a, b)
+
+
 @pytest.mark.parametrize("n_time", [64, 65, 66, 127, 128, 129, 2048, 2049, 16385])
 def test_timeline_lengths(gpulib, n_time):
     """Around chunks (64), groups (2048) and pieces (16384); 64 samples do
