@@ -33,6 +33,15 @@ __device__ __noinline__ bool cx_df_gather(const GatherArgs &a, int det, int t) {
 
 template <int C, int P>
 __device__ __noinline__ void cx_exact_gather(const GatherArgs &a, int det, int t) {
+    if constexpr (P == PX_HP_NT || P == PX_HP_T) {
+        int pix[1][3], n;
+        float pf[3];
+        if (cx_exact_spin<C, P>(a, det, t, pix[0], n, pf)) {
+            const float w[1] = {1.f};
+            gather_taps<P, 1>(a, a.signal + det * a.sig_stride + t, n, pix, w, pf);
+            return;
+        }
+    }
     exact_gather<C, P>(a, det, t, load_quat(a.dets + 4LL * det), __ldg(a.resp + 2 * det),
                        __ldg(a.resp + 2 * det + 1));
 }

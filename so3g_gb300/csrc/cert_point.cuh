@@ -1010,6 +1010,38 @@ __device__ __forceinline__ void cx_for_each(const CxList &list, const CxList &ne
     }
 }
 
+// A HEALPix sample whose spin factors were not certain: its pixel (n taps, 0
+// or 1) from the double-float pointing and only the spin factors in float64;
+// false where the pixel is not certain.  (400 det x 500k, nside 1024, to_map and
+// from_map: 6.9 -> 6.5 ms, the float64 pixel with its divisions left out.  A flat
+// map's float64 pixel is two table lookups, and this made its calls 3 % slower:
+// they take the whole float64 path.)
+template <int C, int P, class Args>
+__device__ __forceinline__ bool cx_exact_spin(const Args &a, int det, int t, int *pix, int &n,
+                                              float (&pf)[3]) {
+    const QuatD ofs = load_quat(a.dets + 4LL * det), b = load_quat(a.bore + 4LL * t);
+    const dfl qd[4] = {df_of(ofs.a), df_of(ofs.b), df_of(ofs.c), df_of(ofs.d)};
+    const float T = __ldg(a.resp + 2 * det), Pr = __ldg(a.resp + 2 * det + 1);
+    dfl qb[4];
+    if (!(df_split(b.a, qb[0]) & df_split(b.b, qb[1]) & df_split(b.c, qb[2]) &
+          df_split(b.d, qb[3])))
+        return false;
+    int px[1][3];
+    float w[1];
+    n = 0;
+    if (!fast_pointing<C, P, false>(a.g, a.ft, a.fc, qb, qd, a.g.ncomp, T, Pr, px, w, n, pf))
+        return false;
+    pix[0] = px[0][0];
+    pix[1] = px[0][1];
+    pix[2] = px[0][2];
+    if (n == 0) return true;
+    // (The coordinates themselves, and their tables, are not used.)
+    double coords[4];
+    get_coords<C>(a.g.lut, b, ofs, coords);
+    spin_factors(a.g.ncomp, coords, T, Pr, pf);
+    return true;
+}
+
 constexpr unsigned kCxFixBlocks = 152 * 8;   // of kBlock threads, striding over a list
 
 // Chunks of a warp's group for a block that has n: even shares for its warps,

@@ -44,10 +44,31 @@ __device__ __noinline__ bool cx_df_sample(const ScatterArgs &a, int det, int t) 
 
 template <int C, int P, bool WEIGHT>
 __device__ __noinline__ void cx_exact_sample(const ScatterArgs &a, int det, int t) {
-    int mult[WEIGHT ? 6 : 3];
+    constexpr int NV = WEIGHT ? 6 : 3;
+    int mult[NV];
     const unsigned vmask = value_slots<WEIGHT>(a.g.ncomp, mult);
     const float T = __ldg(a.resp + 2 * det), Pr = __ldg(a.resp + 2 * det + 1);
     const float wt = a.det_weights ? __ldg(a.det_weights + det) : 1.f;
+    if constexpr (P == PX_HP_NT || P == PX_HP_T) {
+        int pix[3], n;
+        float pf[3];
+        if (cx_exact_spin<C, P>(a, det, t, pix, n, pf)) {
+            if (n == 0) return;
+            long long off, plane;
+            const int bad = locate<P>(a.g, pix, &off, &plane);
+            if (bad >= 0) {
+                record_missing_tile(a.err, bad);
+                return;
+            }
+            const float sig = WEIGHT ? 0.f : __ldg(a.signal + det * a.sig_stride + t);
+            float v[NV];
+            tap_values<WEIGHT, NV, true>(sig, pf, 1.f, wt, v);
+#pragma unroll
+            for (int k = 0; k < NV; k++)
+                if ((vmask >> k) & 1u) atomicAdd(a.map + off + mult[k] * plane, f2d(v[k]));
+            return;
+        }
+    }
     exact_sample<C, P, WEIGHT>(a, det, t, load_quat(a.dets + 4LL * det), T, Pr, wt, mult, vmask);
 }
 
