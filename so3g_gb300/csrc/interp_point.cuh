@@ -44,6 +44,7 @@
 #pragma once
 
 #include "mx_common.cuh"
+#include "pair32.cuh"
 
 namespace so3g {
 
@@ -84,8 +85,8 @@ struct IxBore {
 // Per (detector, chunk): the model's coefficients and bounds, read by the
 // lanes of a chunk (six 16-byte words).
 struct __align__(16) IxParams {
-    float xf, yf, b1, b2;       // x = xb + xf + s (b1 + s (b2 + s b3)) (pixels)
-    float b3, e1, e2, e3;       // y = yb + yf + s (e1 + s (e2 + s e3))
+    float xf, yf, b1, e1;       // x = xb + xf + s (b1 + s (b2 + s b3)) (pixels)
+    float b2, e2, b3, e3;       // y = yb + yf + s (e1 + s (e2 + s e3)), side by side (f32x2)
     float v0r, v0i, v1r, v1i;   // v = v0 + s (v1 + s (v2 + s v3))
     float v2r, v2i, hx, hy;     // hx, hy: 1/2 - bounds (pixels; < 0: not modelled)
     float v3r, v3i, inv_len;    // inv_len = 1 / (tb - ta)
@@ -98,10 +99,10 @@ struct __align__(16) IxParams {
 // the reference's float64 values; the pixel follows from them per sample
 // (hp_pixel_f32).
 struct __align__(16) IxParamsHp {
-    float lon_a, b1, b2, b3;    // lon = lon_a + s (b1 + s (b2 + s b3))
-    float z_a, z1, z2, elon;    // z = z_a + s (z1 + s (z2 + s z3)); elon < 0: not modelled
+    float lon_a, z_a, b1, z1;   // lon = lon_a + s (b1 + s (b2 + s b3))
+    float b2, z2, b3, z3;       // z = z_a + s (z1 + s (z2 + s z3))
     float v0r, v0i, v1r, v1i;   // v as IxParams
-    float v2r, v2i, ez, z3;
+    float v2r, v2i, ez, elon;   // elon < 0: not modelled
     float v3r, v3i, inv_len;
     int ta;
     int pad0, pad1, pad2, pad3;
@@ -222,7 +223,7 @@ __device__ __forceinline__ void ix_setup(const Args &a, const IxBore *ixb, int j
     }
     p.ta = ta;
     p.inv_len = tb > ta ? 1.f / (float)(tb - ta) : 0.f;
-    p.hx = p.hy = -1.f;   // HP: elon = z1 = -1 (the slot's third word of P1)
+    p.hx = p.hy = -1.f;
     IxParamsHp &ph = reinterpret_cast<IxParamsHp &>(p);
     if (HP) ph.elon = -1.f;
     const double2 lo = __ldg(reinterpret_cast<const double2 *>(a.bore + 4LL * ta));
@@ -459,6 +460,14 @@ __device__ __forceinline__ void ix_setup(const Args &a, const IxBore *ixb, int j
     p.hy = 0.5f - by;
 }
 
+// The two cubics held side by side in the first two words, at s (s2: in both
+// halves).
+__device__ __forceinline__ void ix_cubic(f32x2 s2, const float4 *w, float &x, float &y) {
+    const float4 A = w[0], B = w[1];
+    f2_get(f2_fma(s2, f2_fma(s2, f2_fma(s2, f2_make(B.z, B.w), f2_make(B.x, B.y)),
+                             f2_make(A.z, A.w)), f2_make(A.x, A.y)), x, y);
+}
+
 // One sample of a modelled chunk at s = (t - ta) / (tb - ta) (computed by
 // the caller as (float)(t - ta) * inv_len: within 2u of s): pixel (key =
 // iy * nx + ix, on = on the map) and the spin factors of an NC-component
@@ -473,9 +482,10 @@ template <int P, int NC>
 __device__ __forceinline__ bool ix_eval(const IxParams &p, float s, const DGeom &g, float T,
                                         float Pr, int &key, bool &on, float (&pf)[3]) {
     const float4 *w = reinterpret_cast<const float4 *>(&p);
-    const float4 P0 = w[0], P1 = w[1], P3 = w[3], P5 = w[5];
-    const float x = fmaf(s, fmaf(s, fmaf(s, P1.x, P0.w), P0.z), P0.x);
-    const float y = fmaf(s, fmaf(s, fmaf(s, P1.w, P1.z), P1.y), P0.y);
+    const float4 P3 = w[3], P5 = w[5];
+    const f32x2 s2 = f2_both(s);
+    float x, y;
+    ix_cubic(s2, w, x, y);
     const float fxl = floorf(x), fyl = floorf(y);
     const bool ok = (fabsf((x - fxl) - 0.5f) < P3.z) & (fabsf((y - fyl) - 0.5f) < P3.w);
     int ix = __float_as_int(P5.x) + (int)fxl, iy = __float_as_int(P5.y) + (int)fyl;
@@ -492,8 +502,9 @@ __device__ __forceinline__ bool ix_eval(const IxParams &p, float s, const DGeom 
         pf[1] = pf[2] = 0.f;
     } else {
         const float4 P2 = w[2], P4 = w[4];
-        const float vr = fmaf(s, fmaf(s, fmaf(s, P4.x, P3.x), P2.z), P2.x);
-        const float vi = fmaf(s, fmaf(s, fmaf(s, P4.y, P3.y), P2.w), P2.y);
+        float vr, vi;
+        f2_get(f2_fma(s2, f2_fma(s2, f2_fma(s2, f2_make(P4.x, P4.y), f2_make(P3.x, P3.y)),
+                                 f2_make(P2.z, P2.w)), f2_make(P2.x, P2.y)), vr, vi);
         const float k = Pr * rcp_approx(fmaf(vr, vr, vi * vi));
         const float v1 = fmaf(vr, vr, -vi * vi) * k, v2 = 2.f * vr * vi * k;
         if constexpr (NC == 2) {
@@ -516,20 +527,22 @@ template <int P, int NC>
 __device__ __forceinline__ bool ix_eval_hp(const IxParams &pr, float s, const DGeom &g, float T,
                                            float Pr, int &key, float (&pf)[3]) {
     const float4 *w = reinterpret_cast<const float4 *>(&pr);
-    const float4 P0 = w[0], P1 = w[1], P3 = w[3];
-    const float lon = fmaf(s, fmaf(s, fmaf(s, P0.w, P0.z), P0.y), P0.x);
-    const float z = fmaf(s, fmaf(s, fmaf(s, P3.w, P1.z), P1.y), P1.x);
+    const float4 P3 = w[3];
+    const f32x2 s2 = f2_both(s);
+    float lon, z;
+    ix_cubic(s2, w, lon, z);
     int pix[1] = {0};
     const bool ok =
-        P1.w >= 0.f && hp_pixel_f32<P, P == PX_HP_T, true>(g, lon, P1.w, z, P3.z, 0.f, 0.f, pix);
+        P3.w >= 0.f && hp_pixel_f32<P, P == PX_HP_T, true>(g, lon, P3.w, z, P3.z, 0.f, 0.f, pix);
     key = pix[0];
     if constexpr (NC == 1) {
         pf[0] = T;
         pf[1] = pf[2] = 0.f;
     } else {
         const float4 P2 = w[2], P4 = w[4];
-        const float vr = fmaf(s, fmaf(s, fmaf(s, P4.x, P3.x), P2.z), P2.x);
-        const float vi = fmaf(s, fmaf(s, fmaf(s, P4.y, P3.y), P2.w), P2.y);
+        float vr, vi;
+        f2_get(f2_fma(s2, f2_fma(s2, f2_fma(s2, f2_make(P4.x, P4.y), f2_make(P3.x, P3.y)),
+                                 f2_make(P2.z, P2.w)), f2_make(P2.x, P2.y)), vr, vi);
         const float k = Pr * rcp_approx(fmaf(vr, vr, vi * vi));
         const float v1 = fmaf(vr, vr, -vi * vi) * k, v2 = 2.f * vr * vi * k;
         if constexpr (NC == 2) {
