@@ -22,7 +22,7 @@ tensors too.  Every call runs the CUDA kernels: there is no CPU path.
 import ctypes
 import gc
 import os
-import threading
+
 import weakref
 
 import numpy as np
@@ -79,17 +79,9 @@ _TORCH = {"float64": torch.float64, "float32": torch.float32, "int32": torch.int
 _initialized = set()
 
 
-_available = False
-
-
 def _device():
-    # (A call asks several times; is_available() reads the environment anew
-    # each time, 3 us of the ~100 us a small call spends on the host.)
-    global _available
-    if not _available:
-        _available = torch.cuda.is_available()
-        if not _available:
-            raise _abi.LibraryError("so3g_gb300 needs a CUDA device (none is visible)")
+    if not torch.cuda.is_available():
+        raise _abi.LibraryError("so3g_gb300 needs a CUDA device (none is visible)")
     return torch.device("cuda", torch.cuda.current_device())
 
 
@@ -197,10 +189,7 @@ class _ErrRecord:
         return self.t.data_ptr()
 
     def raise_if_set(self):
-        self._raise(*(int(v) for v in self.t.cpu()))
-
-    @staticmethod
-    def _raise(code, a, b, c):
+        code, a, b, c = (int(v) for v in self.t.cpu())
         if code == _abi.DEVERR_MISSING_TILE:
             raise tiling_error(INT32_MAX - a,
                                "Attempted pointing operation on non-instantiated tile.")
@@ -209,38 +198,6 @@ class _ErrRecord:
                              "sample %d)." % (a, b, c))
         if code != 0:
             raise RuntimeError("device error record %d" % code)
-
-
-class _CallErr(_ErrRecord):
-    """The error record of one synchronous call.  Records that a call found
-    clean go back to a small pool of the thread (per device) and need no
-    clearing: a call then pays for the read-back alone, through page-locked
-    memory, which is also its wait for the kernels.  A record that holds an
-    error, or whose call did not get as far as the read-back, is dropped."""
-
-    _pool = threading.local()
-    _POOL_MAX = 4
-
-    def __init__(self):
-        dev = _device()
-        self._free = self._pool.__dict__.setdefault(dev.index, [])
-        if self._free:
-            self.t, self._host = self._free.pop()
-        else:
-            self.t = torch.zeros(4, dtype=torch.int32, device=dev)
-            self._host = torch.empty(4, dtype=torch.int32, pin_memory=True)
-        # (A dropped record's memory waits for this stream's kernels.)
-        self.t.record_stream(torch.cuda.current_stream())
-
-    def raise_if_set(self):
-        self._host.copy_(self.t, non_blocking=True)
-        torch.cuda.current_stream().synchronize()
-        values = self._host.tolist()
-        if not any(values):
-            if len(self._free) < self._POOL_MAX:
-                self._free.append((self.t, self._host))
-            return
-        self._raise(*values)
 
 
 # ---------------------------------------------------------------------------
@@ -1047,7 +1004,7 @@ class ProjEngBase:
         resp = as_array(response, "response", "float32", (n_det, 2))
         bore, dets, resp = self._up((bore, "float64"), (dets, "float64"), (resp, "float32"))
         m.upload()
-        err = _CallErr()
+        err = _ErrRecord()
         lib, pz = _abi.lib(), self._pz()
 
         def launch(d0, d1, buf):
@@ -1089,7 +1046,7 @@ class ProjEngBase:
         bore, dets, resp, w = self._up((bore, "float64"), (dets, "float64"),
                                        (resp, "float32"), (w, "float32"))
         m.upload()
-        err = _CallErr()
+        err = _ErrRecord()
         lib, pz = _abi.lib(), self._pz()
         acc = DEFAULT_ACCUM if accum is None else accum
         host = _host_matrix(sig) if not rng.given else None
@@ -1127,7 +1084,7 @@ class ProjEngBase:
                                        (resp, "float32"), (w, "float32"))
         m.upload()
         rng.upload()
-        err = _CallErr()
+        err = _ErrRecord()
         _abi.check(_abi.lib().so3g_proj_to_weight_map(
             self._pz(), bore.data_ptr(), n_time, dets.data_ptr(), n_det, resp.data_ptr(),
             _ptr(w), rng.ptr(), m.struct, DEFAULT_ACCUM if accum is None else accum,
@@ -1237,7 +1194,7 @@ class ProjEngPrecompBase:
         self._upload(pix, sp)
         m.upload(g)
         sig.upload()
-        err = _CallErr()
+        err = _ErrRecord()
         _abi.check(_abi.lib().so3g_precomp_from_map(
             g, pix.dev.data_ptr(), sp.dev.data_ptr(), n_det, n_time, m.struct,
             sig.dev.data_ptr(), sig.det_stride, err.ptr, _stream()), "precomp from_map")
@@ -1259,7 +1216,7 @@ class ProjEngPrecompBase:
         sig.upload()
         rng.upload()
         w = None if w is None else to_device(w, "float32")
-        err = _CallErr()
+        err = _ErrRecord()
         _abi.check(_abi.lib().so3g_precomp_to_map(
             g, pix.dev.data_ptr(), sp.dev.data_ptr(), n_det, n_time, sig.dev.data_ptr(),
             sig.det_stride, _ptr(w), rng.ptr(), m.struct,
@@ -1280,7 +1237,7 @@ class ProjEngPrecompBase:
         m.upload(g)
         rng.upload()
         w = None if w is None else to_device(w, "float32")
-        err = _CallErr()
+        err = _ErrRecord()
         _abi.check(_abi.lib().so3g_precomp_to_weight_map(
             g, pix.dev.data_ptr(), sp.dev.data_ptr(), n_det, n_time, _ptr(w), rng.ptr(),
             m.struct, DEFAULT_ACCUM if accum is None else accum, err.ptr, _stream()),
