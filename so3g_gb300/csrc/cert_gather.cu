@@ -11,7 +11,8 @@
 //
 // Bound by instruction issue.  CAR TQU 3 x 2000 x 2000, 1000 det x 1M
 // samples: 30.9 -> 8.4 ms, and with the steps that two quantities or two
-// samples share as f32x2 instructions 7.7 ms (of which 1.3 ms the fallback).
+// samples share as f32x2 instructions 7.7 ms; with models for the longer side
+// of the turn-arounds 7.3 ms (of which 0.9 ms the fallback).
 
 #include "cert_point.cuh"
 #include "cert_map.cuh"
@@ -137,7 +138,7 @@ __global__ void __launch_bounds__(kCxBlock, kCxGatherBlocks)
             const float4 w3 = w[3];
             const float kq = (float)(tq - __float_as_int(w3.z));
             float res[4][3];
-            if (NC > 1 && w3.w != 0.f) cx_residuals(model.resid, tq, res);
+            if (w3.w != 0.f) cx_residuals(model.resid, tq, res);
             unsigned f4 = 0u;
             // (In the whole warp: not a piece's end or an odd last chunk.)
             const bool full = (g + 2 * r + 2) * kCxLen <= t1 && 2 * r + 2 <= nch;

@@ -20,7 +20,9 @@
 // that fits every sample to ~1e-13, else (time stamps and encoders jitter)
 // the quadratic through its first, middle and last sample, with the
 // residual of each sample kept as a small rotation rho, q(t) = Q (1 + rho),
-// in 3 x 16 bits.
+// in 3 x 16 bits.  A chunk with a break (the turn-around of a triangle scan) gets
+// the quadratic of the break's longer side; the samples of the other are
+// marked and go to the per-sample path.
 //
 // With A(u) = Q(u) q_det, alpha = a + i d and beta = c + i b are polynomials
 // in u, alpha = alpha_0 (1 + z_1 u + z_2 u^2 + ...), and so are, to the order
@@ -60,6 +62,10 @@ constexpr int kCxWarps = kCxBlock / 32;
 // 5.7 against 2.8).
 constexpr float kCxRough = 6e-7f;
 
+// The first residual word of a sample its chunk's model does not cover (the
+// others' are within 32001).
+constexpr int kCxUncovered = -32768;
+
 // Classes of coordinate systems the models are compiled for.
 enum { CX_CAR = 0, CX_ZEN = 1 };
 
@@ -70,7 +76,7 @@ struct __align__(16) CxBore {
     float e;               // max |q(t) - Q|
     float eta;             // max ||q(t)|^2 - 1|
     float lsb;             // residuals' unit; 0: none kept (e is negligible)
-    float pad;
+    float part;            // 1: some samples are not covered (residuals kCxUncovered)
 };
 
 // The boresight models of a call: per chunk, and the residuals per sample.
@@ -179,16 +185,86 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
     eta = max_parts(eta);
     // 1e-13: the double-float roundings.
     const float E4 = sqrtf(sum4(r4 * r4)) * 1.00001f + 1e-13f;
-    const float E2 = sqrtf(sum4(r2 * r2)) * 1.00001f + 1e-13f;
+    float E2 = sqrtf(sum4(r2 * r2)) * 1.00001f + 1e-13f;
     const bool quad = !(E4 < 2.5e-13f);
+    // A chunk that holds a break (a turn-around): its largest second
+    // difference is there, and the longer side of it gets a quadratic of its
+    // own (through its ends and middle, written about the chunk's middle): a
+    // turn-around every 20 s had sent 1.6 % of a scan's samples to the
+    // per-sample path, 0.78 ms of 1000 det x 1M samples; now 0.35 ms.
+    dfl q0 = q[2], p1 = b1, p2 = b2;
+    int c0 = k0, c1 = k1;   // samples covered
+    const bool broken = quad && !bad && !(E2 < kCxRough);
+    if (__any_sync(kFull, broken)) {
+        int top = 0;   // magnitude (float bits), its low bits the sample
+        for (int n = 0; n < kCxLen / 4; n++) {
+            const int k = min(max(k0 + part * (kCxLen / 4) + n, 1), min(k1, kCxLen - 1));
+            const float d = (float)((__ldg(b + 4 * (k + 1)) - __ldg(b + 4 * k)) -
+                                    (__ldg(b + 4 * k) - __ldg(b + 4 * (k - 1))));
+            top = max(top, (__float_as_int(fabsf(d)) & ~127) | k);
+        }
+#pragma unroll
+        for (int m = 1; m < 16; m <<= 1) top = max(top, __shfl_xor_sync(kFull, top, m));
+        const int s = top & 127;
+        int A = s + 1, B = k1;
+        if (s - 1 - k0 > k1 - s - 1) {
+            A = k0;
+            B = s - 1;
+        }
+        if ((B - A) & 1) {   // (an even length, without the sample at the break)
+            if (A == k0) B--;
+            else A++;
+        }
+        const bool fit = broken && B - A >= 16;
+        const int M = fit ? (A + B) >> 1 : kCxMid, H = fit ? (B - A) >> 1 : kCxMid;
+        dfl x[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) df_split(__ldg(b + 4 * (M + (k - 1) * H)), x[k]);
+        const float al = (float)kCxLen / (float)H, de = (float)(kCxMid - M) / (float)H;
+        const dfl o = df_mulf(df_sub(x[2], x[0]), 0.5f);
+        const dfl e = df_mulf(df_sub(df_add(x[0], x[2]), df_mulf(x[1], 2.f)), 0.5f);
+        dfl w0 = df_add(x[1], df_mulf(df_add(o, df_mulf(e, de)), de));
+        dfl w1 = df_mulf(df_add(o, df_mulf(e, 2.f * de)), al);
+        dfl w2 = df_mulf(df_mulf(e, al), al);
+        // To norm 1 at the chunk's middle, which may lie outside the side (the
+        // spin factors there are taken for a unit quaternion; the pixel's bound
+        // has the rest).
+        dfl nn = df_mul(w0, w0);
+        nn = df_add(nn, dfl{__shfl_xor_sync(kFull, nn.hi, 1), __shfl_xor_sync(kFull, nn.lo, 1)});
+        nn = df_add(nn, dfl{__shfl_xor_sync(kFull, nn.hi, 2), __shfl_xor_sync(kFull, nn.lo, 2)});
+        const float off = df_sub(nn, dfl{1.f, 0.f}).hi, sc = -0.5f * off;
+        w0 = df_add(w0, df_mulf(w0, sc));
+        w1 = df_add(w1, df_mulf(w1, sc));
+        w2 = df_add(w2, df_mulf(w2, sc));
+        float r = 0.f;
+        for (int n = 0; n < kCxLen / 4; n++) {
+            const int k = fit ? min(max(k0 + part * (kCxLen / 4) + n, A), B) : kCxMid;
+            dfl v;
+            df_split(__ldg(b + 4 * k), v);
+            const float u = (float)(k - kCxMid) * (1.f / kCxLen);
+            r = fmaxf(r, fabsf(df_sub(df_sub(v, w0), df_mulf(df_add(w1, df_mulf(w2, u)), u)).hi));
+        }
+        r = max_parts(r);
+        r = sqrtf(sum4(r * r)) * 1.00001f + 1e-13f;
+        // (Noise without a break does not fit any side much better.)
+        if (fit && fabsf(off) < 1e-5f && r < 0.1f * E2) {
+            E2 = r;
+            eta = fmaxf(eta, off * off + 1e-13f);
+            q0 = w0;
+            p1 = w1;
+            p2 = w2;
+            c0 = A;
+            c1 = B;
+        }
+    }
     const float lsb = quad && !bad ? E2 * (1.f / 32000.f) : 0.f;
     if (chunk < n_chunks && part == 0) {
         float *o = reinterpret_cast<float *>(out + j);
-        o[comp] = q[2].hi;
-        o[4 + comp] = q[2].lo;
-        o[8 + comp] = quad ? b1.hi : a1.hi;
-        o[12 + comp] = quad ? b1.lo : a1.lo;
-        o[16 + comp] = quad ? b2.hi : a2.hi;
+        o[comp] = q0.hi;
+        o[4 + comp] = q0.lo;
+        o[8 + comp] = quad ? p1.hi : a1.hi;
+        o[12 + comp] = quad ? p1.lo : a1.lo;
+        o[16 + comp] = quad ? p2.hi : a2.hi;
         o[20 + comp] = quad ? 0.f : a3;
         o[24 + comp] = quad ? 0.f : a4;
         if (comp == 0) {
@@ -196,6 +272,7 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
             out[j].e = bad ? 1.f : (quad ? E2 : E4);
             out[j].eta = bad ? 1.f : eta * 1.00001f + 1e-14f;
             out[j].lsb = lsb;
+            out[j].part = c0 > k0 || c1 < k1 ? 1.f : 0.f;
         }
     }
     // Residuals: rho = conj(Q) (q - Q), in units of lsb.
@@ -207,8 +284,8 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
         dfl v;
         df_split(__ldg(b + 4 * kc), v);
         const float u = (float)(kc - kCxMid) * (1.f / kCxLen);
-        const dfl p2 = df_mulf(df_add(b1, df_mulf(b2, u)), u);
-        const float r = df_sub(df_sub(v, q[2]), p2).hi * inv, g = v.hi;
+        const dfl p = df_mulf(df_add(p1, df_mulf(p2, u)), u);
+        const float r = df_sub(df_sub(v, q0), p).hi * inv, g = v.hi;
         float rr[4], qq[4];
 #pragma unroll
         for (int c = 0; c < 4; c++) {
@@ -219,8 +296,10 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
             const float x = qq[0] * rr[1] - qq[1] * rr[0] - qq[2] * rr[3] + qq[3] * rr[2];
             const float y = qq[0] * rr[2] + qq[1] * rr[3] - qq[2] * rr[0] - qq[3] * rr[1];
             const float z = qq[0] * rr[3] - qq[1] * rr[2] + qq[2] * rr[1] - qq[3] * rr[0];
-            resid[base + k] = make_short4((short)__float2int_rn(x), (short)__float2int_rn(y),
-                                          (short)__float2int_rn(z), 0);
+            resid[base + k] = k < c0 || k > c1
+                                  ? make_short4((short)kCxUncovered, 0, 0, 0)
+                                  : make_short4((short)__float2int_rn(x), (short)__float2int_rn(y),
+                                                (short)__float2int_rn(z), 0);
         }
     }
 }
@@ -370,7 +449,9 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
     w[3] = make_float4(0.f, 0.f, __int_as_float(mid), 0.f);
     const CxBore &cb = cxb[j];
     const float E = __ldg(&cb.e), lsb = __ldg(&cb.lsb);
-    if (!(E < 1e-6f)) return;
+    // (A side's norm may be off by E, which the bilinear form does not cover.)
+    const bool covered = __ldg(&cb.part) == 0.f;
+    if (!(E < 1e-6f) || (BL && !covered)) return;
     // The middle sample: its coordinates X0, Y0 (HEALPix: longitude and
     // sin(lat)) and spin quantities, certified double-float.
     dfl qa, qb, qc, qe, X0, Y0, Nc, Ns, D;
@@ -692,7 +773,7 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         w[1] = make_float4(cx2 * icx * s2, cy2 * icy * s2, cx3 * icx * s3, cy3 * icy * s3);
     }
     float e = 0.f;
-    bool flag = BL && lsb > 0.f;
+    bool flag = (BL && lsb > 0.f) || !covered;
     if constexpr (SPIN) {
         // The spin factors at the middle, F1 + i F2 = P v^2 / D, and phi's
         // derivative there, 2 (Im(alpha_1 conj(alpha_0)) / |alpha_0|^2 + ...
@@ -865,11 +946,12 @@ __device__ __forceinline__ bool cx_sample(const float4 *w, f32x2 k2, const float
     const f32x2 xy =
         f2_fma(k2, f2_fma(k2, f2_fma(k2, cx_hi(P1), cx_lo(P1)), cx_hi(P0)), cx_lo(P0));
     bool ok;
+    const bool left = flag && res[0] < (float)(kCxUncovered + 200);
     if constexpr (P == PX_HP_NT || P == PX_HP_T) {
         float x, y;
         f2_get(xy, x, y);
         key = cx_hp_pixel<P>((int)g.nside, g.nest, (int)g.npix, x, P2.x, y, P2.y);
-        ok = key >= 0;
+        ok = (key >= 0) & !left;
         on = true;
     } else {
         const float4 P3 = w[3];
@@ -879,7 +961,7 @@ __device__ __forceinline__ bool cx_sample(const float4 *w, f32x2 k2, const float
         float rx, ry, dx, dy;
         f2_get(r2, rx, ry);
         f2_get(f2_sub(xy, f2_sub(r2, magic)), dx, dy);
-        ok = (fabsf(dx) < P2.x) & (fabsf(dy) < P2.y);
+        ok = (fabsf(dx) < P2.x) & (fabsf(dy) < P2.y) & !left;
         int ix = __float_as_int(P3.x) + __float_as_int(rx),
             iy = __float_as_int(P3.y) + __float_as_int(ry);
         if constexpr (P == PX_FLAT_T_NN) {

@@ -15,8 +15,8 @@
 // Bound by instruction issue (~200 warp-instructions per 32 samples, the
 // per-sample path ~910), then by the L2 atomic units.  CAR TQU 3 x 2000 x
 // 2000, 1000 det x 1M samples: to_map 26.2 -> 8.3 ms, with f32x2 instructions
-// for the coordinates, the spin factors and the runs' sums 8.0 ms (of which
-// 1.2 ms the fallback), to_weight_map of 500 x 500k 7.3 -> 2.8 ms; HEALPix
+// for the coordinates, the spin factors and the runs' sums 8.0 ms, with models
+// for the longer side of the turn-arounds 7.9 ms (of which 0.75 ms the fallback), to_weight_map of 500 x 500k 7.3 -> 2.8 ms; HEALPix
 // nside 1024, 400 det x 500k, to_map + from_map 15.6 -> 5.6 ms.
 #pragma once
 
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(kCxBlock, CxScatterBlocks<WEIGHT>::value)
             const float4 w3 = w[3];
             const float kq = (float)(tq - __float_as_int(w3.z));
             float res[4][3];
-            if (NC > 1 && w3.w != 0.f) cx_residuals(model.resid, tq, res);
+            if (w3.w != 0.f) cx_residuals(model.resid, tq, res);
             const float sg[4] = {sc.x, sc.y, sc.z, sc.w};
             int key[4];
             float pf[4][3];

@@ -146,6 +146,16 @@ def test_rough_boresight(gpulib, geom, t0, noise):
     _check_all(p.get_ProjEng("TQU"), args, rng)
 
 
+@pytest.mark.parametrize("comps", ["T", "TQU"])
+@pytest.mark.parametrize("geom", ["CAR", "ZEA", "HP-RING"])
+@pytest.mark.parametrize("n_time", [4449, 4481])
+def test_turn_arounds_everywhere(gpulib, geom, comps, n_time):
+    """A turn-around every 67 samples: at every offset within a chunk, and in
+    the last chunk, of one sample or of 33."""
+    p, args, rng = _inputs(geom, 4, n_time, el=45., throw=67 / 200.)
+    _check_all(p.get_ProjEng(comps), args, rng)
+
+
 @pytest.mark.parametrize("geom", ["CAR", "CAR-tiled"])
 def test_ranges_and_weights(gpulib, geom):
     """Ranges starting and ending anywhere, overlapping, some empty."""
