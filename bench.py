@@ -282,12 +282,13 @@ class ClockSampler:
 # DRAM bytes per sample (dram__bytes_read.sum + dram__bytes_write.sum / samples)
 # of one ncu capture of the to_map and from_map kernels, CAR TQU 3x2000x2000,
 # 200 det x 1M samples, per pointing mode (profiles/to_map_from_map_*_car_
-# tqu_200det_1M.md; mixed: the chunked main kernels k_scatter_ix4 and
-# k_from_map_ix4).  The traffic is the signal (4 B read, from_map also 4 B
-# written) and the boresight per detector, so it scales with the samples.
+# tqu_200det_1M.md; the chunked main kernels: mixed k_scatter_ix4 and
+# k_from_map_ix4, certified k_scatter_cx and k_from_map_cx).  The traffic is
+# the signal (4 B read, from_map also 4 B written) and the boresight per
+# detector, so it scales with the samples.
 MEASURED_TRAFFIC_PER_SAMPLE = {
-    "certified": {"to_map": (834.33e6 + 3.78e6) / 2e8,
-                  "from_map": (835.40e6 + 747.14e6) / 2e8},
+    "certified": {"to_map": (811.80e6 + 16.89e6) / 2e8,
+                  "from_map": (813.74e6 + 952.03e6) / 2e8},
     "mixed": {"to_map": (807.045e6 + 13.405e6) / 2e8,
               "from_map": (806.769e6 + 790.061e6) / 2e8},
 }

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kBlock) k_from_map_cx_fix(const __grid_constan
                 [&](int det, int t) { cx_exact_gather<C, P>(a, det, t); });
 }
 
-constexpr int kCxGatherBlocks = 6;   // resident blocks per SM (80 registers; 8: 3 % slower)
+constexpr int kCxGatherBlocks = 6;   // resident blocks per SM (80 registers; 5 and 7 the same, 8: 3 % slower)
 
 template <int CL, int P, int NC>
 __global__ void __launch_bounds__(kCxBlock, kCxGatherBlocks)

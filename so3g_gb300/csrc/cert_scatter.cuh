@@ -284,9 +284,9 @@ __device__ __forceinline__ bool cx_runs4(const ScatterArgs &a, CxRuns<NV> &rb, i
     return true;
 }
 
-// Resident blocks per SM: 24 warps with 80 registers (to_map; 32 warps with
-// 64, more spills, took 5 % longer, 40 another 15 %), 20 (to_weight_map, whose
-// held-back runs take more shared memory).
+// Resident blocks per SM: 20 warps with 96 registers (to_map: 7.9 ms for 1000
+// det x 1M samples; 24 warps with 80, more spills, 9.1 ms), 16 (to_weight_map,
+// whose held-back runs take more shared memory; 20: 2 % slower).
 template <bool WEIGHT>
 struct CxScatterBlocks {
     static constexpr int value = WEIGHT ? 4 : 5;
