@@ -36,7 +36,10 @@
 // The spin factors are expanded to u^4, their u^1 coefficient in
 // double-float, the pixel coordinates to u^3; the terms left out are
 // bounded by the majorant series of the logarithms and the exponential
-// (cx_tail5; ~1e-13 on the 1 deg/s scans of the workloads).  The residual
+// (cx_tail_log, cx_tail_exp; ~1e-13 on the 1 deg/s scans of the workloads).
+// The latitude and the modulus of CAR's spin factors also depend on the
+// quaternions' norm, which the reference does not divide out: the bounds take
+// it from the chunk's samples and the detector (eta, spread).  The residual
 // turns the spin factors' phase phi by grad(phi) . rho, the gradient a linear
 // function of u per chunk and detector, and moves the pixel by at most
 // 2 |rho| / cos(lat), which goes into the pixel's bound.
@@ -75,8 +78,10 @@ struct __align__(16) CxBore {
     float4 a2, a3, a4;
     float e;               // max |q(t) - Q|
     float eta;             // max ||q(t)|^2 - 1|
+    float spread;          // max ||q(t)|^2 - |Q(0)|^2|
     float lsb;             // residuals' unit; 0: none kept (e is negligible)
     float part;            // 1: some samples are not covered (residuals kCxUncovered)
+    float pad[3];
 };
 
 // The boresight models of a call: per chunk, and the residuals per sample.
@@ -154,7 +159,15 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
     const dfl b1 = o2, b2 = df_mulf(e2, 2.f);
     const int k0 = j * kCxLen - base;                        // first own sample
     const int k1 = min(kCxLen - 1 + k0, n_time - 1 - base);  // last own sample
-    float r4 = 0.f, r2 = 0.f, eta = 0.f;
+    // |q|^2 - 1 of one sample, from the four components' lanes.
+    auto norm1 = [](const dfl &v) {
+        dfl s = df_mul(v, v);
+        s = df_add(s, dfl{__shfl_xor_sync(kFull, s.hi, 1), __shfl_xor_sync(kFull, s.lo, 1)});
+        s = df_add(s, dfl{__shfl_xor_sync(kFull, s.hi, 2), __shfl_xor_sync(kFull, s.lo, 2)});
+        return df_sub(s, dfl{1.f, 0.f}).hi;
+    };
+    float r4 = 0.f, r2 = 0.f;
+    float top_n = norm1(q[2]), low_n = top_n;   // largest and smallest |q|^2 - 1
     for (int n = 0; n < kCxLen / 4; n++) {   // (the same count in every lane)
         const int k = min(k0 + part * (kCxLen / 4) + n, k1);
         dfl v;
@@ -166,10 +179,9 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
         const dfl p2 = df_mulf(df_add(b1, df_mulf(b2, u)), u);
         r4 = fmaxf(r4, fabsf(df_sub(d, p4).hi));   // (fmaxf drops NaN: only a bad
         r2 = fmaxf(r2, fabsf(df_sub(d, p2).hi));   // value makes one)
-        dfl s = df_mul(v, v);
-        s = df_add(s, dfl{__shfl_xor_sync(kFull, s.hi, 1), __shfl_xor_sync(kFull, s.lo, 1)});
-        s = df_add(s, dfl{__shfl_xor_sync(kFull, s.hi, 2), __shfl_xor_sync(kFull, s.lo, 2)});
-        eta = fmaxf(eta, fabsf(df_sub(s, dfl{1.f, 0.f}).hi));
+        const float n1 = norm1(v);
+        top_n = fmaxf(top_n, n1);
+        low_n = fminf(low_n, n1);
     }
     bad = __any_sync(kFull, bad);   // (the warp's other chunk as well)
     auto max_parts = [](float x) {
@@ -182,7 +194,9 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
     };
     r4 = max_parts(r4);
     r2 = max_parts(r2);
-    eta = max_parts(eta);
+    top_n = max_parts(top_n);
+    low_n = -max_parts(-low_n);
+    float eta = fmaxf(fabsf(top_n), fabsf(low_n)), spread = top_n - low_n;
     // 1e-13: the double-float roundings.
     const float E4 = sqrtf(sum4(r4 * r4)) * 1.00001f + 1e-13f;
     float E2 = sqrtf(sum4(r2 * r2)) * 1.00001f + 1e-13f;
@@ -226,9 +240,8 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
         dfl w0 = df_add(x[1], df_mulf(df_add(o, df_mulf(e, de)), de));
         dfl w1 = df_mulf(df_add(o, df_mulf(e, 2.f * de)), al);
         dfl w2 = df_mulf(df_mulf(e, al), al);
-        // To norm 1 at the chunk's middle, which may lie outside the side (the
-        // spin factors there are taken for a unit quaternion; the pixel's bound
-        // has the rest).
+        // To norm 1 (within off^2) at the chunk's middle, which may lie outside
+        // the side.
         dfl nn = df_mul(w0, w0);
         nn = df_add(nn, dfl{__shfl_xor_sync(kFull, nn.hi, 1), __shfl_xor_sync(kFull, nn.lo, 1)});
         nn = df_add(nn, dfl{__shfl_xor_sync(kFull, nn.hi, 2), __shfl_xor_sync(kFull, nn.lo, 2)});
@@ -250,6 +263,7 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
         if (fit && fabsf(off) < 1e-5f && r < 0.1f * E2) {
             E2 = r;
             eta = fmaxf(eta, off * off + 1e-13f);
+            spread = eta + off * off;
             q0 = w0;
             p1 = w1;
             p2 = w2;
@@ -271,6 +285,7 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
             if (bad || (quad && !(E2 < kCxRough))) atomicAdd(rough, 1u);
             out[j].e = bad ? 1.f : (quad ? E2 : E4);
             out[j].eta = bad ? 1.f : eta * 1.00001f + 1e-14f;
+            out[j].spread = bad ? 1.f : spread * 1.00001f + 1e-14f;
             out[j].lsb = lsb;
             out[j].part = c0 > k0 || c1 < k1 ? 1.f : 0.f;
         }
@@ -449,6 +464,13 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
     w[3] = make_float4(0.f, 0.f, __int_as_float(mid), 0.f);
     const CxBore &cb = cxb[j];
     const float E = __ldg(&cb.e), lsb = __ldg(&cb.lsb);
+    // The norm of q(t) q_det: its distance from 1, and from the middle's.
+    float eta, spread;
+    {
+        const dfl qq = df_dot<4>(qd, qd);
+        eta = __ldg(&cb.eta) + fabsf((qq.hi - 1.f) + qq.lo);
+        spread = 1.01f * __ldg(&cb.spread);
+    }
     // (A side's norm may be off by E, which the bilinear form does not cover.)
     const bool covered = __ldg(&cb.part) == 0.f;
     if (!(E < 1e-6f) || (BL && !covered)) return;
@@ -509,6 +531,7 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
     float lutx = 0.f, luty = 0.f;    // the tables' errors at both ends
     float zz;                        // |z1|^2 of alpha and beta
     float gerr;                      // gradient of phi: error of its linear form
+    float mod = 0.f;                 // spin factors' modulus: change over the chunk (relative)
     cf x4{0.f, 0.f};                 // BL: the u^4 coefficient of Y - i X
     if constexpr (CL == CX_CAR) {
         if (!(be2 > 0.004f)) return;
@@ -557,13 +580,23 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
             cy3 = C * (m3 - S * m1 * m2 + (S * S - C2) * (1.f / 6.f) * m1 * m1 * m1);
         }
         rx = 1.05f * ra * rb;
-        ry = 2.1f;
+        ry = 2.2f;
         // h^2/8 max|f''| of the tables: ATAN2 3.0e-10, ASIN 4.66e-10 S (1 -
         // S^2)^-3/2 (at an S beyond the chunk's); the middle's and the sample's.
         const float zs = fminf(fabsf(S) + 1.1f * C * mu, 0.9985f);
         const float rs = rsqrtf(1.f - zs * zs);
         lutx = 2.f * 3.1e-10f;
         luty = (HP ? 1.f : 2.f) * 4.7e-10f * zs * rs * rs * rs;
+        // The norm N = |alpha|^2 + |beta|^2: the reference's sin(lat) is N
+        // tanh(ln|alpha / beta|), so a sample's N off the middle's by up to
+        // `spread` moves it by spread |tanh|, and the coefficients above, which
+        // take C^2 for 1 - S^2 (it is N^2 - S^2) and N for 1, are off by up to 5
+        // eta / (1 - S^2) of their terms (eta <= 1e-3 here, 1 - S^2 > 0.016).  (A
+        // residual moves ln|alpha / beta| by 2 E / C.)
+        const float ms = mu + 2.2f * E * rs;
+        ty += (1.1f * spread * zs + 5.f * eta * ms) * (HP ? 1.f : rs);
+        // The spin factors' modulus is (N^2 - S^2) / (1 - S^2), not 1.
+        mod = rs * rs * (2.2f * spread + 5.f * eta * zs * ms);
         // The longitude stays inside (-pi, pi) over the chunk (a HEALPix pixel
         // takes it modulo 2 pi).
         if (!HP && !(fabsf(X0.hi) + 1.05f * (ta.X + tb.X) + rx * E + 1e-6f < 3.1415f)) return;
@@ -598,7 +631,8 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
             e3 = z3 + g1 * z2 + g2 * z1 + cf{g3, 0.f};
             g *= ic;
             h += 2.4f * f * ta.X;
-            rx = 2.4f * ic * ic;
+            // (2 ic^2 for a turn, 2 ic^2 sin(theta) for a change of norm.)
+            rx = 2.9f * ic * ic;
         } else if (coord == SO3G_COORD_ZEA) {
             const float t1 = la.l1.i, t2 = la.l2.i, t3 = la.l3.i;
             e1 = cf{0.f, t1};
@@ -837,19 +871,16 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         w[6] = make_float4(o[0][4], o[1][4], o[0][5], o[1][5]);
         w[7] = make_float4(o[0][6], o[1][6], 0.f, 0.f);
         // e: the double-float error and the reference's roundings (kEpsPf;
-        // phi1's is of the same size), the terms left out, a norm off 1
-        // (CAR's reference divides by (1 - sin^2) / 4, the model by
-        // |alpha beta|^2), the float32 errors of phi2 (16u |z1|^2), phi3,
+        // phi1's is of the same size), the terms left out, the modulus'
+        // change, the float32 errors of phi2 (16u |z1|^2), phi3,
         // phi4 and of the products, the correction's roundings (3u of its
         // terms), and the boresight's distance from Q.
         const float h1 = 0.5f * fabsf(p1), h2 = 0.25f * fabsf(phi2) + u * zz,
                     h3 = 0.125f * fabsf(phi3) + 8.f * u * zz, h4 = 0.0625f * fabsf(phi4) + 8.f * u * zz;
         const CxTail tp = cx_tail(h1, h2, h3, h4);
         const float Df = D.hi;
-        const dfl qq = df_dot<4>(qd, qd);
-        const float eta = __ldg(&cb.eta) + fabsf((qq.hi - 1.f) + qq.lo);
         e = 1.2f * (cx_tail_exp(tp) + 4.f * tail) +
-            kEpsPf * fmaxf(1.f, 0.25f / Df) * (1.f + h1) + (CL == CX_CAR ? 0.6f * eta / Df : 0.f) +
+            kEpsPf * fmaxf(1.f, 0.25f / Df) * (1.f + h1) + 1.1f * mod +
             u * (3.f * h1 * h1 + 8.f * h2 + 4.f * zz + 16.f * (h3 + h4 + h1 * (h2 + h1 * h1)));
         e = e * fmaxf(aP, 1e-3f) + 3.f * u * 18.f * gr;
         if (lsb > 0.f) {
