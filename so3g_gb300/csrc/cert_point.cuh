@@ -17,12 +17,14 @@
 //
 // The boresight of a chunk is modelled by a polynomial Q(u) (u = (t - tm) /
 // 64, tm its middle sample): the quartic through five of its samples where
-// that fits every sample to ~1e-13, else (time stamps and encoders jitter)
+// that fits every sample to 1.5e-13, else (time stamps and encoders jitter)
 // the quadratic through its first, middle and last sample, with the
 // residual of each sample kept as a small rotation rho, q(t) = Q (1 + rho),
 // in 3 x 16 bits.  A chunk with a break (the turn-around of a triangle scan) gets
 // the quadratic of the break's longer side; the samples of the other are
-// marked and go to the per-sample path.
+// marked and go to the per-sample path.  (rho is the vector part of conj(q)
+// (q - Q); the scalar part, a change of norm, turns nothing: it goes into the
+// bilinear form's bound, and through the samples' norm into the pixel's.)
 //
 // With A(u) = Q(u) q_det, alpha = a + i d and beta = c + i b are polynomials
 // in u, alpha = alpha_0 (1 + z_1 u + z_2 u^2 + ...), and so are, to the order
@@ -81,7 +83,8 @@ struct __align__(16) CxBore {
     float spread;          // max ||q(t)|^2 - |Q(0)|^2|
     float lsb;             // residuals' unit; 0: none kept (e is negligible)
     float part;            // 1: some samples are not covered (residuals kCxUncovered)
-    float pad[3];
+    float rho0;            // max |Re(conj(q) (q - Q))|, the residuals' part that is no turn
+    float pad[2];
 };
 
 // The boresight models of a call: per chunk, and the residuals per sample.
@@ -287,6 +290,7 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
             out[j].eta = bad ? 1.f : eta * 1.00001f + 1e-14f;
             out[j].spread = bad ? 1.f : spread * 1.00001f + 1e-14f;
             out[j].lsb = lsb;
+            if (!(lsb > 0.f)) out[j].rho0 = out[j].e;
             out[j].part = c0 > k0 || c1 < k1 ? 1.f : 0.f;
         }
     }
@@ -294,6 +298,7 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
     if (!__any_sync(kFull, lsb > 0.f)) return;
     const float inv = lsb > 0.f ? 1.f / lsb : 0.f;
     const int lane0 = threadIdx.x & 28;
+    float rho0 = 0.f;   // in units of lsb
     for (int n = 0; n < kCxLen / 4; n++) {
         const int k = k0 + part * (kCxLen / 4) + n, kc = min(k, k1);
         dfl v;
@@ -307,6 +312,9 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
             rr[c] = __shfl_sync(kFull, r, lane0 + c);
             qq[c] = __shfl_sync(kFull, g, lane0 + c);
         }
+        if (kc >= c0 && kc <= c1)
+            rho0 = fmaxf(rho0, fabsf(qq[0] * rr[0] + qq[1] * rr[1] + qq[2] * rr[2] +
+                                     qq[3] * rr[3]));
         if (comp == (k & 3) && k <= k1 && chunk < n_chunks && inv > 0.f) {
             const float x = qq[0] * rr[1] - qq[1] * rr[0] - qq[2] * rr[3] + qq[3] * rr[2];
             const float y = qq[0] * rr[2] + qq[1] * rr[3] - qq[2] * rr[0] - qq[3] * rr[1];
@@ -317,6 +325,10 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
                                                 (short)__float2int_rn(z), 0);
         }
     }
+    rho0 = max_parts(rho0);
+    // (0.1 lsb: the sums' float32 roundings, 8u of 32000.)
+    if (chunk < n_chunks && part == 0 && comp == 0 && lsb > 0.f)
+        out[j].rho0 = (rho0 + 0.1f) * lsb;
 }
 
 // Complex float32.
@@ -532,7 +544,8 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
     float zz;                        // |z1|^2 of alpha and beta
     float gerr;                      // gradient of phi: error of its linear form
     float mod = 0.f;                 // spin factors' modulus: change over the chunk (relative)
-    cf x4{0.f, 0.f};                 // BL: the u^4 coefficient of Y - i X
+    cf x4{0.f, 0.f};                 // BL: the u^4 coefficient of Y - i X,
+    float xs = 2.f;                  // and X, Y's change with the norm of q (relative)
     if constexpr (CL == CX_CAR) {
         if (!(be2 > 0.004f)) return;
         const float ib = rcp_approx(be2);
@@ -630,6 +643,7 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
             e2 = z2 + g1 * z1 + cf{g2, 0.f};
             e3 = z3 + g1 * z2 + g2 * z1 + cf{g3, 0.f};
             g *= ic;
+            xs = 2.f * ic;
             h += 2.4f * f * ta.X;
             // (2 ic^2 for a turn, 2 ic^2 sin(theta) for a change of norm.)
             rx = 2.9f * ic * ic;
@@ -639,6 +653,7 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
             e2 = cf{-0.5f * t1 * t1, t2};
             e3 = cf{-t1 * t2, t3 - (1.f / 6.f) * t1 * t1 * t1};
             g *= rsqrtf(al2);
+            xs = 1.f;
             rx = 2.4f * ia;
         } else {
             e1 = z1;
@@ -773,11 +788,15 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         const float y2 = cy2 * icy * s2, y3 = cy3 * icy * s3, y4p = x4.r * icy * s4;
         // Errors: the terms left out, the corrections' float32 roundings and
         // those of the coefficients (12u of their terms), the residual's
-        // second order and quantisation, its gradient's linear form.
+        // second order and quantisation, its gradient's linear form, and
+        // the residual's part that is no turn: it scales q, and X and Y with it
+        // (SIN 2, ZEA 1, TAN 2 / cos(theta) times their size).
         const float cor = 1024.f * (fabsf(cx2 * icx) + fabsf(cy2 * icy)) * s2 +
                           32768.f * (fabsf(cx3 * icx) + fabsf(cy3 * icy)) * s3 + 2e-4f;
         const float ai = fmaxf(aix, aiy);
+        const float far = fmaxf(fabsf(X0.hi), fabsf(Y0.hi)) + fmaxf(sx, sy);
         const float eb = tx * ai + 12.f * u * cor + 3e-12f * rx * ai +
+                         1.2f * xs * far * __ldg(&cb.rho0) * ai +
                          (lsb > 0.f ? rx * ai * (E * (16.f * E + 2.f * zz + 32.f * u) + 2.f * lsb)
                                     : rx * ai * E);
         if (!(eb < kCxBlPix && (sx * aix + 1.f) < 60.f && (sy * aiy + 1.f) < 60.f)) return;
