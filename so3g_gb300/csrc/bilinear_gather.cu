@@ -1,23 +1,22 @@
-// bilinear_gather.cu -- from_map of untiled bilinear TAN, ZEA and SIN maps with
-// the chunked pointing of cert_point.cuh (its bilinear form), in the mixed and
-// the certified mode.
+// bilinear_gather.cu -- from_map of untiled bilinear TAN, ZEA and SIN maps in
+// the mixed mode with the chunked pointing of cert_point.cuh (its bilinear
+// form).
 //
 // A bilinear weight needs the fraction of the pixel coordinate to float32
 // accuracy, so the coordinates are held as the spin factors are, an exact
 // float32 part plus a correction (within kCxBlPix of the reference's), and the
-// weights formed from the fraction in double-float: the floats nearest the
-// reference's weights or their neighbours, as the per-sample paths' are.  The
-// terms are float32 sums over the float32 map copy (mixed) or certified
-// roundings of the reference's float64 sums (certified).  (CAR's coordinates
-// come from interpolation tables, whose kinks the chunk models do not
-// follow to that accuracy: it keeps the per-sample kernels; so does to_map,
+// weights formed from the fraction in double-float; the terms are float32 sums
+// over the float32 map copy.  The certified mode keeps the per-sample kernels:
+// its weights are the floats nearest the double-float coordinates' weights,
+// which a float32 correction does not give in every last bit.  (CAR's
+// coordinates come from interpolation tables, whose kinks the chunk models do
+// not follow to that accuracy: it keeps the per-sample kernels; so does to_map,
 // whose float64 sums keep the per-sample weights to the last bit.)
 //
 // Bound by instruction issue: the per-sample kernel ~850 warp-instructions
-// per 32 samples (3000 x 3000 ZEA map of 0.5' pixels, 400 det x 300k, mixed: 2.9
-// -> 1.2 ms; with f32x2 instructions the same, within 1 %).
+// per 32 samples (3000 x 3000 ZEA map of 0.5' pixels, 400 det x 300k: 2.9 -> 1.2
+// ms; with f32x2 instructions the same, within 1 %).
 
-#include "cert_map.cuh"
 #include "cert_point.cuh"
 #include "gather_kernel.cuh"
 
@@ -27,13 +26,12 @@ namespace {
 
 // One sample the models left: the double-float pointing (false: not
 // certain), the float64 pointing.
-template <int C, bool CERT>
+template <int C>
 __device__ __noinline__ bool bl_df_sample(const GatherArgs &a, int det, int t) {
     const QuatD ofs = load_quat(a.dets + 4LL * det);
     const dfl qd[4] = {df_of(ofs.a), df_of(ofs.b), df_of(ofs.c), df_of(ofs.d)};
-    const float T = __ldg(a.resp + 2 * det), Pr = __ldg(a.resp + 2 * det + 1);
-    if (CERT) return df_gather_cert<C, PX_FLAT_NT_BL>(a, det, t, qd, T, Pr);
-    return df_gather<C, PX_FLAT_NT_BL>(a, det, t, qd, T, Pr);
+    return df_gather<C, PX_FLAT_NT_BL>(a, det, t, qd, __ldg(a.resp + 2 * det),
+                                       __ldg(a.resp + 2 * det + 1));
 }
 
 template <int C>
@@ -42,17 +40,17 @@ __device__ __noinline__ void bl_exact_sample(const GatherArgs &a, int det, int t
                                    __ldg(a.resp + 2 * det), __ldg(a.resp + 2 * det + 1));
 }
 
-template <int C, bool CERT>
+template <int C>
 __device__ __noinline__ void bl_any_sample(const GatherArgs &a, int det, int t) {
-    if (!bl_df_sample<C, CERT>(a, det, t)) bl_exact_sample<C>(a, det, t);
+    if (!bl_df_sample<C>(a, det, t)) bl_exact_sample<C>(a, det, t);
 }
 
-template <int C, bool CERT, int TIER>
+template <int C, int TIER>
 __global__ void __launch_bounds__(kBlock) k_from_map_bl_fix(const __grid_constant__ GatherArgs a,
                                                             CxList list, CxList next) {
     cx_for_each(list, next,
                 [&](int det, int t) -> bool {
-                    if (TIER == 0) return bl_df_sample<C, CERT>(a, det, t);
+                    if (TIER == 0) return bl_df_sample<C>(a, det, t);
                     bl_exact_sample<C>(a, det, t);
                     return true;
                 },
@@ -69,11 +67,9 @@ __device__ __forceinline__ bool bl_floor(float S, float L, float e, int base, in
     return (d.hi > e) & (d.hi < 1.f - e);
 }
 
-template <int NC, bool CERT>
+template <int NC>
 __global__ void __launch_bounds__(kCxBlock, 5)
-    k_from_map_bl(const __grid_constant__ GatherArgs a, CxModel model, CxList left, int coord,
-                  const float4 *cmap) {
-    constexpr int W = CxMap<NC, false>::W;
+    k_from_map_bl(const __grid_constant__ GatherArgs a, CxModel model, CxList left, int coord) {
     __shared__ float4 s_model[kCxWarps][kCxGroup][kCxBlWords];
     __shared__ CxWarp s_warp[kCxWarps];
     int det, t0, t1;
@@ -97,9 +93,9 @@ __global__ void __launch_bounds__(kCxBlock, 5)
     const int ny = a.g.ny, nx = a.g.nx;
     auto over = [&](int t) {
         switch (coord) {
-        case SO3G_COORD_TAN: bl_any_sample<SO3G_COORD_TAN, CERT>(a, det, t); break;
-        case SO3G_COORD_ZEA: bl_any_sample<SO3G_COORD_ZEA, CERT>(a, det, t); break;
-        default: bl_any_sample<SO3G_COORD_SIN, CERT>(a, det, t); break;
+        case SO3G_COORD_TAN: bl_any_sample<SO3G_COORD_TAN>(a, det, t); break;
+        case SO3G_COORD_ZEA: bl_any_sample<SO3G_COORD_ZEA>(a, det, t); break;
+        default: bl_any_sample<SO3G_COORD_SIN>(a, det, t); break;
         }
     };
     const int j0 = t0 / kCxLen, j1 = (t1 - 1) / kCxLen + 1;
@@ -162,12 +158,7 @@ __global__ void __launch_bounds__(kCxBlock, 5)
                     f32x2 S, Lp;
                     float v1, v2;
                     cx_factors(w, k2, res[i], w3.w != 0.f, S, Lp);
-                    if (CERT) {
-                        const bool c = cx_round(S, Lp, cx_hi(W9), v1, v2);
-                        ok = ok & (c | !on);
-                    } else {
-                        f2_get(f2_add(S, Lp), v1, v2);
-                    }
+                    f2_get(f2_add(S, Lp), v1, v2);
                     pf[NC - 2] = v1;
                     pf[NC - 1] = v2;
                 }
@@ -186,28 +177,13 @@ __global__ void __launch_bounds__(kCxBlock, 5)
                             if (xx < 0 || xx >= nx) continue;
                             const float wt = df_mul(wy[dy], wx[dx]).hi;
                             const long long off = (long long)yy * nx + xx;
-                            if constexpr (!CERT) {
-                                const float4 m = __ldg(a.map32 + off);
-                                s = fmaf(m.x, pf[0] * wt, s);
-                                if constexpr (NC > 1) s = fmaf(m.y, pf[1] * wt, s);
-                                if constexpr (NC > 2) s = fmaf(m.z, pf[2] * wt, s);
-                            } else {
-                                float hl[4 * W];
-#pragma unroll
-                                for (int q = 0; q < W; q++) {
-                                    const float4 m = __ldg(cmap + off * W + q);
-                                    hl[4 * q] = m.x;
-                                    hl[4 * q + 1] = m.y;
-                                    hl[4 * q + 2] = m.z;
-                                    hl[4 * q + 3] = m.w;
-                                }
-#pragma unroll
-                                for (int c = 0; c < NC; c++)
-                                    ok = ok & cx_accum(s, hl[2 * c], hl[2 * c + 1], pf[c], wt);
-                            }
+                            const float4 m = __ldg(a.map32 + off);
+                            s = fmaf(m.x, pf[0] * wt, s);
+                            if constexpr (NC > 1) s = fmaf(m.y, pf[1] * wt, s);
+                            if constexpr (NC > 2) s = fmaf(m.z, pf[2] * wt, s);
                         }
                     }
-                    if (ok) sv[i] = s;
+                    sv[i] = s;
                 }
                 if (!ok) f4 |= 1u << i;
             }
@@ -226,52 +202,32 @@ __global__ void __launch_bounds__(kCxBlock, 5)
     cx_append(cw, left, det, over);
 }
 
-template <int C, bool CERT>
+template <int C>
 int bl_fix(const GatherArgs &a, const CxWork &w, cudaStream_t st) {
-    k_from_map_bl_fix<C, CERT, 0><<<kCxFixBlocks, kBlock, 0, st>>>(a, w.left, w.exact);
+    k_from_map_bl_fix<C, 0><<<kCxFixBlocks, kBlock, 0, st>>>(a, w.left, w.exact);
     const int rc = after_launch("bilinear fallback");
     if (rc != SO3G_OK) return rc;
-    k_from_map_bl_fix<C, CERT, 1><<<kCxFixBlocks, kBlock, 0, st>>>(a, w.exact, w.exact);
+    k_from_map_bl_fix<C, 1><<<kCxFixBlocks, kBlock, 0, st>>>(a, w.exact, w.exact);
     return after_launch("bilinear fallback (exact)");
 }
 
-template <int NC, bool CERT>
-int bl_run(const GatherArgs &a, const CxWork &w, int coord, long long npix, dim3 grid,
-           cudaStream_t st) {
-    float4 *cmap = nullptr;
-    if (CERT) {
-        constexpr int W = CxMap<NC, false>::W;
-        if (cudaMallocAsync(reinterpret_cast<void **>(&cmap), sizeof(float4) * W * (size_t)npix,
-                            st) != cudaSuccess) {
-            cudaGetLastError();
-            return 1;
-        }
-        k_cx_map<PX_FLAT_NT_NN, NC><<<(unsigned)((npix + kBlock - 1) / kBlock), kBlock, 0, st>>>(
-            a.g, a.map, npix, cmap);
-        const int rc = after_launch("bilinear from_map (map copy)");
-        if (rc != SO3G_OK) {
-            cudaFreeAsync(cmap, st);
-            return rc;
-        }
-    }
-    k_from_map_bl<NC, CERT><<<grid, kCxBlock, 0, st>>>(a, w.model, w.left, coord, cmap);
+template <int NC>
+int bl_run(const GatherArgs &a, const CxWork &w, int coord, dim3 grid, cudaStream_t st) {
+    k_from_map_bl<NC><<<grid, kCxBlock, 0, st>>>(a, w.model, w.left, coord);
     const int rc = after_launch("bilinear from_map (chunked)");
-    if (cmap) cudaFreeAsync(cmap, st);
     if (rc != SO3G_OK) return rc;
     switch (coord) {
-    case SO3G_COORD_TAN: return bl_fix<SO3G_COORD_TAN, CERT>(a, w, st);
-    case SO3G_COORD_ZEA: return bl_fix<SO3G_COORD_ZEA, CERT>(a, w, st);
-    default: return bl_fix<SO3G_COORD_SIN, CERT>(a, w, st);
+    case SO3G_COORD_TAN: return bl_fix<SO3G_COORD_TAN>(a, w, st);
+    case SO3G_COORD_ZEA: return bl_fix<SO3G_COORD_ZEA>(a, w, st);
+    default: return bl_fix<SO3G_COORD_SIN>(a, w, st);
     }
 }
 
-template <bool CERT>
-int bl_nc(const GatherArgs &a, const CxWork &w, int coord, long long npix, dim3 grid,
-          cudaStream_t st) {
+int bl_nc(const GatherArgs &a, const CxWork &w, int coord, dim3 grid, cudaStream_t st) {
     switch (a.g.ncomp) {
-    case 1: return bl_run<1, CERT>(a, w, coord, npix, grid, st);
-    case 2: return bl_run<2, CERT>(a, w, coord, npix, grid, st);
-    default: return bl_run<3, CERT>(a, w, coord, npix, grid, st);
+    case 1: return bl_run<1>(a, w, coord, grid, st);
+    case 2: return bl_run<2>(a, w, coord, grid, st);
+    default: return bl_run<3>(a, w, coord, grid, st);
     }
 }
 
@@ -280,24 +236,19 @@ int bl_nc(const GatherArgs &a, const CxWork &w, int coord, long long npix, dim3 
 int chunked_bilinear_from_map(int coord, int kind, GatherArgs &args, int n_det, cudaStream_t st,
                               void **work) {
     GatherArgs a = args;
-    const bool cert = a.fast == SO3G_POINTING_CERTIFIED;
-    const bool mixed = a.fast == SO3G_POINTING_MIXED && a.map32;
     const bool zen = coord == SO3G_COORD_TAN || coord == SO3G_COORD_ZEA || coord == SO3G_COORD_SIN;
     const long long npix = (long long)a.g.ny * a.g.nx;
     const long long n_time = a.segs.n_time, samples = n_time * n_det;
-    const long long least = cert_chunked_min_samples();
-    // (The certified map copy must pay for itself, as in cert_from_map.)
-    if (!(cert || mixed) || kind != PX_FLAT_NT_BL || !zen || n_time <= kCxLen || npix <= 0 ||
-        npix >= (1LL << 31) || samples < least ||
-        (cert && (npix > (1LL << 28) || (least > 0 && 2 * (samples - least) < npix))))
+    if (a.fast != SO3G_POINTING_MIXED || !a.map32 || kind != PX_FLAT_NT_BL || !zen ||
+        n_time <= kCxLen || npix <= 0 || npix >= (1LL << 31) ||
+        samples < cert_chunked_min_samples())
         return 1;
     CxWork w;
     if (!cx_work(w, a.bore, (int)n_time, samples, st)) return 1;
     a.piece = cx_piece(n_det, n_time);
     a.gate = w.gate;
     const dim3 grid((unsigned)n_det, (unsigned)((n_time + a.piece - 1) / a.piece));
-    const int rc = cert ? bl_nc<true>(a, w, coord, npix, grid, st)
-                        : bl_nc<false>(a, w, coord, npix, grid, st);
+    const int rc = bl_nc(a, w, coord, grid, st);
     if (rc != SO3G_OK) {
         cudaFreeAsync(w.mem, st);
         return rc;

@@ -1,5 +1,5 @@
 // cert_map.cuh -- the certified chunked from_map's copy of the map and its
-// certified float32 accumulation (cert_gather.cu, bilinear_gather.cu).
+// certified float32 accumulation (cert_gather.cu).
 #pragma once
 
 #include "host.h"
@@ -127,27 +127,6 @@ __device__ __forceinline__ bool cx_accum_all(float sig, const float (&hl)[4 * W]
     float r;
     const bool ok = cx_accum_slow<NC, W>(sig, m0, m1, pf[0], pf[1], pf[2], &r);
     out = r;
-    return ok;
-}
-
-// The same for a bilinear tap of weight w: sig + m * pf * w as the reference's
-// two float64 products and sum.
-__device__ __forceinline__ bool cx_accum(float &sig, float h, float l, float pf, float w) {
-    const float p0 = h * pf;
-    const float pe = fmaf(l, pf, fmaf(h, pf, -p0));
-    const float p = p0 * w;
-    const float q = fmaf(pe, w, fmaf(p0, w, -p));
-    float S, x;
-    two_sum(sig, p, S, x);
-    const float L = x + q, e = 5e-13f * (fabsf(p) + fabsf(sig));
-    float r = S + (L + e);
-    bool ok = (r == S + (L - e)) & (fabsf(r) > 1e-30f);
-    if (!ok && (h == 0.f || ((pf == 0.f || w == 0.f) && h == h))) {
-        r = sig + __int_as_float((__float_as_int(h) ^ __float_as_int(pf) ^ __float_as_int(w)) &
-                                 0x80000000);
-        ok = true;
-    }
-    if (ok) sig = r;
     return ok;
 }
 

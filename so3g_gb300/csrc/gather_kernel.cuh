@@ -24,7 +24,7 @@ struct GatherArgs {
     MixedConst mc;
     const float4 *bore32;   // float32 boresight (mixed pointing), or NULL
     const float4 *map32;    // float32 (T, Q, U, 0) per pixel (mixed pointing), or NULL
-    SkipIf gate;            // certified pointing: the kernel's gate, or none
+    SkipIf gate;            // the kernel's gate beside a chunked one, or none
 };
 
 // The chunked certified from_map (cert_gather.cu) of n_det whole detectors;
@@ -32,9 +32,8 @@ struct GatherArgs {
 // cert_to_map (scatter_kernel.cuh).
 int cert_from_map(int coord, int kind, GatherArgs &args, int n_det, cudaStream_t st,
                   void **work);
-// The chunked from_map with untiled bilinear TAN, ZEA and SIN maps, certified
-// or mixed (bilinear_gather.cu; mixed: args.map32 must be set); as
-// cert_from_map.
+// The chunked from_map with untiled bilinear TAN, ZEA and SIN maps in the mixed
+// mode (bilinear_gather.cu; args.map32 must be set); as cert_from_map.
 int chunked_bilinear_from_map(int coord, int kind, GatherArgs &args, int n_det, cudaStream_t st,
                               void **work);
 

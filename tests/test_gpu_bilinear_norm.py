@@ -16,6 +16,7 @@ import pytest
 import so3g_gb300 as so3g
 from so3g_gb300 import _abi, synth
 from so3g_gb300.proj import quat
+from conftest import bits_equal
 from test_gpu_cert_chunked import _both
 
 pytestmark = pytest.mark.gpu
@@ -44,21 +45,36 @@ def _scan(boresight):
     return q
 
 
-@pytest.mark.parametrize("boresight", ["unit", "float32", "noise", "accelerating"])
-@pytest.mark.parametrize("proj", ["TAN", "ZEA", "SIN"])
-def test_residual_norm(gpulib, proj, boresight):
+def _call(proj, boresight):
+    """(engine, map, arguments): a checkerboard of 0.5 arcmin pixels."""
     import torch
     k = np.arange(N_DET)
     r, a = 1. * DEG * np.sqrt((k + .5) / N_DET), 2.4 * k
     dets = np.asarray(quat.rotation_xieta(r * np.cos(a), r * np.sin(a), 0.7 * k))
     resp = np.ones((N_DET, 2), np.float32)
     args = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (_scan(boresight), dets, resp)]
-    ny, nx = 1201, 1502       # 0.5 arcmin pixels
+    ny, nx = 1201, 1502
     eng = getattr(so3g, "ProjEng_%s_T_NonTiled_Bilinear" % proj)(
         (ny, nx, .5 * synth.ARCMIN, -.5 * synth.ARCMIN, ny / 2. + .5, nx / 2. + .5))
-    eng.pointing = _abi.POINTING_MIXED
     yx = torch.arange(ny, device="cuda")[:, None] + torch.arange(nx, device="cuda")
-    m = (1. - 2. * (yx % 2)).double()[None].contiguous()
+    return eng, (1. - 2. * (yx % 2)).double()[None].contiguous(), args
+
+
+@pytest.mark.parametrize("boresight", ["unit", "float32", "noise", "accelerating"])
+@pytest.mark.parametrize("proj", ["TAN", "ZEA", "SIN"])
+def test_residual_norm(gpulib, proj, boresight):
+    eng, m, args = _call(proj, boresight)
+    eng.pointing = _abi.POINTING_MIXED
     chunked, general = _both(lambda: eng.from_map(m, *args, None))
     assert float((general != 0).float().mean()) > 0.3
     assert float((chunked.double() - general.double()).abs().max()) <= TOL
+
+
+@pytest.mark.parametrize("proj", ["TAN", "ZEA", "SIN"])
+def test_default_mode_weights(gpulib, proj):
+    """In the default mode a weight is the float32 nearest the double-float
+    coordinates' weight at every call size."""
+    eng, m, args = _call(proj, "unit")
+    chunked, general = _both(lambda: eng.from_map(m, *args, None))
+    assert float((general != 0).float().mean()) > 0.3
+    assert bits_equal(chunked.cpu().numpy(), general.cpu().numpy())
