@@ -213,8 +213,10 @@ int bl_fix(const GatherArgs &a, const CxWork &w, cudaStream_t st) {
 
 template <int NC>
 int bl_run(const GatherArgs &a, const CxWork &w, int coord, dim3 grid, cudaStream_t st) {
+    int rc = cx_probe<CX_ZEN, false, NC, true>(a, w, coord, grid.x, nullptr, st);
+    if (rc != SO3G_OK) return rc;
     k_from_map_bl<NC><<<grid, kCxBlock, 0, st>>>(a, w.model, w.left, coord);
-    const int rc = after_launch("bilinear from_map (chunked)");
+    rc = after_launch("bilinear from_map (chunked)");
     if (rc != SO3G_OK) return rc;
     switch (coord) {
     case SO3G_COORD_TAN: return bl_fix<SO3G_COORD_TAN>(a, w, st);

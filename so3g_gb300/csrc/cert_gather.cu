@@ -226,9 +226,12 @@ int cx_gather_run(const GatherArgs &a, const CxWork &w, int coord, long long npi
         cudaGetLastError();
         return 1;
     }
-    k_cx_map<P, NC><<<(unsigned)((npix + kBlock - 1) / kBlock), kBlock, 0, st>>>(a.g, a.map, npix,
-                                                                                cmap);
-    int rc = after_launch("from_map (map copy)");
+    int rc = cx_probe<CL, P == PX_HP_NT || P == PX_HP_T, NC, false>(a, w, coord, grid.x, nullptr, st);
+    if (rc == SO3G_OK) {
+        k_cx_map<P, NC><<<(unsigned)((npix + kBlock - 1) / kBlock), kBlock, 0, st>>>(
+            a.g, a.map, npix, cmap, a.gate);
+        rc = after_launch("from_map (map copy)");
+    }
     if (rc == SO3G_OK) {
         k_from_map_cx<CL, P, NC><<<grid, kCxBlock, 0, st>>>(a, w.model, w.left, coord, cmap);
         rc = after_launch("from_map (certified, chunked)");

@@ -20,7 +20,8 @@ struct CxMap {
 // NaN where m is not finite or outside df_split's range (such a sample goes
 // to the float64 path).
 template <int P, int NC>
-__global__ void k_cx_map(DGeom g, const double *map, long long npix, float4 *out) {
+__global__ void k_cx_map(DGeom g, const double *map, long long npix, float4 *out, SkipIf gate) {
+    if (gate.holds()) return;
     constexpr bool TILED = P == PX_FLAT_T_NN || P == PX_HP_T;
     constexpr int W = CxMap<NC, TILED>::W;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;

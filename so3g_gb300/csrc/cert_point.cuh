@@ -59,13 +59,17 @@ constexpr int kCxMid = kCxLen / 2;
 constexpr int kCxGroup = 32;          // chunks of a warp's group, one per lane
 constexpr int kCxBlock = 128;         // threads per block (its warps are independent)
 constexpr int kCxWarps = kCxBlock / 32;
-// A boresight whose residuals exceed this in more than a quarter of its
-// chunks (pointing noise of ~0.03") is not taken: the call's general kernel
-// is faster than sending most samples to the per-sample path (200 det x 500k,
-// to_map: noise of 1e-8 per quaternion component 1.26 ms against 2.83, 1e-7
-// 2.4 on a CAR map and 6.8 on a fast HEALPix scan against 2.8 and 3.4, 1e-6
-// 5.7 against 2.8).
-constexpr float kCxRough = 6e-7f;
+// A chunk that its quadratic misses by more than this is searched for a break.
+constexpr float kCxBreak = 6e-7f;
+// (detector, chunk) models that k_cx_probe looks at.
+constexpr int kCxProbes = 2048;
+// A call whose models would leave more than one sample in this to the
+// per-sample path takes the general kernel.  Up to there the list holds them
+// (200 det x 500k, TQU, to_map / from_map against the general kernel: 7 % left
+// on a CAR map 0.48 / 0.39 of its time, on a HEALPix map 0.57 / 0.47; 10 %
+// 0.92 / 0.78; past the list's end the main kernel handles them in place, 25 %
+// of a T map 1.2 / 1.0, all 2 to 3).
+constexpr unsigned kCxShare = 12;
 
 // The first residual word of a sample its chunk's model does not cover (the
 // others' are within 32001).
@@ -127,6 +131,9 @@ constexpr float kCxBlPix = 2.5e-7f;
 constexpr float kCxMagic = 12582912.f;
 constexpr int kCxMagicBits = 0x4b400000;
 
+// Counters of a call: entries of the two lists, k_cx_probe's votes.
+constexpr int kCxCounts = 4;
+
 // Middle sample of chunk j (samples [64 j, 64 j + 64)); the last chunk's is
 // moved back so that its model's samples mid - 32 .. mid + 32 exist.
 __device__ __forceinline__ int cx_mid(int j, int n_time) {
@@ -138,8 +145,9 @@ __device__ __forceinline__ int cx_mid(int j, int n_time) {
 // arithmetic (the float64 pipe would take ~0.1 ms per million samples).
 __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time, int n_chunks,
                                                  CxBore *out, short4 *resid,
-                                                 unsigned *rough) {
+                                                 unsigned long long *counts) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < kCxCounts) counts[i] = 0;   // (of the kernels that follow)
     const int chunk = i >> 4, j = min(chunk, n_chunks - 1), comp = i & 3, part = (i >> 2) & 3;
     const int base = cx_mid(j, n_time) - kCxMid;
     const double *b = bore + 4LL * base + comp;
@@ -211,7 +219,7 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
     // per-sample path, 0.78 ms of 1000 det x 1M samples; now 0.35 ms.
     dfl q0 = q[2], p1 = b1, p2 = b2;
     int c0 = k0, c1 = k1;   // samples covered
-    const bool broken = quad && !bad && !(E2 < kCxRough);
+    const bool broken = quad && !bad && !(E2 < kCxBreak);
     if (__any_sync(kFull, broken)) {
         int top = 0;   // magnitude (float bits), its low bits the sample
         for (int n = 0; n < kCxLen / 4; n++) {
@@ -285,7 +293,6 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
         o[20 + comp] = quad ? 0.f : a3;
         o[24 + comp] = quad ? 0.f : a4;
         if (comp == 0) {
-            if (bad || (quad && !(E2 < kCxRough))) atomicAdd(rough, 1u);
             out[j].e = bad ? 1.f : (quad ? E2 : E4);
             out[j].eta = bad ? 1.f : eta * 1.00001f + 1e-14f;
             out[j].spread = bad ? 1.f : spread * 1.00001f + 1e-14f;
@@ -932,6 +939,76 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
                        flag ? 1.f : 0.f);
 }
 
+// The share of a modelled chunk's samples that the per-sample path will take
+// (cx_sample finds the pixel or a spin factor's rounding not certain): the
+// bounds against the pixel's size and the spacing of floats at the middle's
+// factors.
+template <bool HP, int NC, bool BL>
+__device__ __forceinline__ float cx_share(const float4 *w, float nside, bool covered) {
+    if constexpr (BL) return w[9].z >= 0.f ? 0.f : 1.f;
+    const float hx = w[2].x, hy = w[2].y;
+    if (HP ? !(hx >= 0.f) : !(hx > 0.f && hy > 0.f)) return 1.f;
+    // (HEALPix: the two in-face indices, nside (4 lon / 2 pi +- 3/4 z) in the
+    // equatorial belt, each within 1.5 times that; a third more for the caps.)
+    float s = HP ? 8.f * nside * (0.64f * hx + 0.75f * hy) : 2.f - 2.f * (hx + hy);
+    if constexpr (NC > 1) {
+        const float e = w[2].z, v[2] = {w[4].x + w[5].x, w[4].y + w[5].y};
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const float ulp = __int_as_float(__float_as_int(v[c]) & 0x7f800000) * 1.1920929e-7f;
+            s += ulp > 0.f ? 2.f * e / ulp : 1.f;
+        }
+    }
+    if (!covered) s += 0.25f;   // (on average, of a chunk with a break)
+    return s < 1.f ? s : 1.f;   // (1 for a NaN)
+}
+
+// Whether the models are worth it: kCxProbes of the call's chunks, spread over
+// its segments and their time, give the share of samples that the models will
+// leave (a rough boresight, quaternions off unit length, a scan over a pole, a
+// detectors without polarisation response) as votes[0] of votes[1]; within a
+// tenth of the share counted on flat maps, a third on HEALPix ones (200 det x
+// 500k, pointing noise of 1e-9 to 1e-7, polar scans, interpolated boresights).
+// One model per lane, 64 warps: a call pays the latency of one set-up.  Without
+// it a boresight or detectors stored in 32 bits, or a scan over the pole, took
+// 2 to 3 times the general kernel's time; now 1.02 to 1.05.
+template <int CL, bool HP, int NC, bool BL, class Args>
+__global__ void __launch_bounds__(32)
+    k_cx_probe(const __grid_constant__ Args a, const CxBore *bore, int coord, int n_seg,
+               const float *det_weights, unsigned long long *votes) {
+    const int i = blockIdx.x * 32 + threadIdx.x;
+    const int s = (int)((long long)i * n_seg / kCxProbes);
+    int det = s, t0 = 0, t1 = a.segs.n_time;
+    if (a.segs.seg) {
+        det = __ldg(a.segs.seg + 3 * s);
+        t0 = __ldg(a.segs.seg + 3 * s + 1);
+        t1 = __ldg(a.segs.seg + 3 * s + 2);
+    }
+    unsigned long long left = 0, all = 0;
+    if (t1 > t0 && !(det_weights && __ldg(det_weights + det) == 0.f)) {
+        const int j0 = t0 / kCxLen, n = (t1 - 1) / kCxLen + 1 - j0;
+        const int j = j0 + (int)__umulhi((unsigned)i * 2654435769u, (unsigned)n);
+        const QuatD ofs = load_quat(a.dets + 4LL * det);
+        const dfl qd[4] = {df_of(ofs.a), df_of(ofs.b), df_of(ofs.c), df_of(ofs.d)};
+        float4 w[BL ? kCxBlWords : kCxWords];
+        cx_setup<CL, HP, NC, BL>(a, bore, coord, j, a.segs.n_time, qd,
+                                 __ldg(a.resp + 2 * det + 1), w);
+        const float share =
+            cx_share<HP, NC, BL>(w, (float)(int)a.g.nside, __ldg(&bore[j].part) == 0.f);
+        all = 1024ULL * (unsigned)n;
+        left = (unsigned long long)(share * 1024.f) * (unsigned)n;
+    }
+#pragma unroll
+    for (int m = 16; m; m >>= 1) {
+        left += __shfl_xor_sync(kFull, left, m);
+        all += __shfl_xor_sync(kFull, all, m);
+    }
+    if (threadIdx.x == 0) {
+        atomicAdd(votes, left);
+        atomicAdd(votes + 1, all);
+    }
+}
+
 __device__ __forceinline__ f32x2 cx_lo(const float4 &w) { return f2_make(w.x, w.y); }
 __device__ __forceinline__ f32x2 cx_hi(const float4 &w) { return f2_make(w.z, w.w); }
 
@@ -1066,7 +1143,8 @@ __device__ __forceinline__ void cx_residuals(const short4 *resid, int t, float (
 // what that leaves to another list, for the float64 path: every path runs
 // on full warps, and the main kernel's code stays small (with the per-sample
 // paths called from it, instruction fetch stalls made it 2.2 times slower).
-// Entries past a list's capacity are handled on the spot.
+// Entries past a list's capacity are handled on the spot; a call that would
+// fill the list takes the general kernel (k_cx_probe).
 
 struct CxList {
     unsigned long long *count;
@@ -1198,13 +1276,13 @@ inline int cx_piece(long long n_seg, long long max_len) {
 }
 
 // The workspace of a call, in stream-ordered memory: the chunks' boresight
-// models, the residuals and the two lists (one entry for every 24 and 96
+// models, the residuals and the two lists (one entry for every 10 and 96
 // samples: the workloads leave 1 in 50 and 1 in 1000).
 struct CxWork {
     void *mem = nullptr;
     CxModel model;
     CxList left, exact;
-    SkipIf gate;               // the chunked kernels skip when it holds
+    SkipIf gate;               // the chunked kernels skip when it holds (after cx_probe)
 };
 
 // Allocates the workspace and makes the boresight models; false (nothing
@@ -1212,7 +1290,7 @@ struct CxWork {
 inline bool cx_work(CxWork &w, const double *bore, int n_time, long long samples,
                     cudaStream_t stream) {
     const long long n_chunks = (n_time + kCxLen - 1) / kCxLen;
-    const long long cap1 = samples / 24 + 4096, cap2 = samples / 96 + 4096;
+    const long long cap1 = samples / 10 + 4096, cap2 = samples / 96 + 4096;
     const size_t o_res = 256 + sizeof(CxBore) * (size_t)n_chunks;
     const size_t o_l1 = o_res + sizeof(short4) * (size_t)(n_chunks * kCxLen);
     const size_t o_l2 = o_l1 + sizeof(int2) * (size_t)cap1;
@@ -1229,23 +1307,25 @@ inline bool cx_work(CxWork &w, const double *bore, int n_time, long long samples
     w.model = CxModel{models, resid};
     w.left = CxList{counts, reinterpret_cast<int2 *>(p + o_l1), (unsigned long long)cap1};
     w.exact = CxList{counts + 1, reinterpret_cast<int2 *>(p + o_l2), (unsigned long long)cap2};
-    unsigned *rough = reinterpret_cast<unsigned *>(counts + 2);
-    w.gate = SkipIf{rough, (unsigned)(n_chunks / 4), true};
-    bool ok = cudaMemsetAsync(counts, 0, 256, stream) == cudaSuccess;
-    if (ok) {
-        const long long threads = 16 * n_chunks;
-        k_cx_bore<<<(unsigned)((threads + 127) / 128), 128, 0, stream>>>(bore, n_time,
-                                                                        (int)n_chunks, models, resid,
-                                                                        rough);
-        ok = after_launch("boresight chunk models (certified)") == SO3G_OK;
-    }
-    if (!ok) {
-        cudaGetLastError();
+    w.gate = SkipIf{counts + 2, kCxShare, true};
+    const long long threads = 16 * n_chunks;
+    k_cx_bore<<<(unsigned)((threads + 127) / 128), 128, 0, stream>>>(
+        bore, n_time, (int)n_chunks, models, resid, counts);
+    if (after_launch("boresight chunk models (certified)") != SO3G_OK) {
         cudaFreeAsync(w.mem, stream);
         w.mem = nullptr;
         clear_error();
+        return false;
     }
-    return ok;
+    return true;
+}
+
+template <int CL, bool HP, int NC, bool BL, class Args>
+int cx_probe(const Args &a, const CxWork &w, int coord, long long n_seg, const float *det_weights,
+             cudaStream_t st) {
+    k_cx_probe<CL, HP, NC, BL><<<kCxProbes / 32, 32, 0, st>>>(
+        a, w.model.bore, coord, (int)n_seg, det_weights, w.left.count + 2);
+    return after_launch("share of samples the chunk models leave");
 }
 
 }  // namespace

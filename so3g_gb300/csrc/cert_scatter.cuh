@@ -442,16 +442,25 @@ int cx_scatter_fix(const ScatterArgs &a, const CxWork &w, cudaStream_t st) {
     return after_launch("certified fallback (exact)");
 }
 
+template <int CL, int P, bool WEIGHT, int NC>
+int cx_scatter_main(const ScatterArgs &a, const CxWork &w, int coord, dim3 grid, cudaStream_t st) {
+    constexpr bool HP = P == PX_HP_NT || P == PX_HP_T;
+    const int rc = cx_probe<CL, HP, NC, false>(a, w, coord, grid.x, a.det_weights, st);
+    if (rc != SO3G_OK) return rc;
+    k_scatter_cx<CL, P, WEIGHT, NC><<<grid, kCxBlock, 0, st>>>(a, w.model, w.left, coord);
+    return after_launch(WEIGHT ? "to_weight_map (certified, chunked)"
+                               : "to_map (certified, chunked)");
+}
+
 template <int CL, int P, bool WEIGHT>
 int cx_scatter_launch(const ScatterArgs &a, const CxWork &w, int coord, dim3 grid,
                       cudaStream_t st) {
+    int rc;
     switch (a.g.ncomp) {
-    case 1: k_scatter_cx<CL, P, WEIGHT, 1><<<grid, kCxBlock, 0, st>>>(a, w.model, w.left, coord); break;
-    case 2: k_scatter_cx<CL, P, WEIGHT, 2><<<grid, kCxBlock, 0, st>>>(a, w.model, w.left, coord); break;
-    default: k_scatter_cx<CL, P, WEIGHT, 3><<<grid, kCxBlock, 0, st>>>(a, w.model, w.left, coord); break;
+    case 1: rc = cx_scatter_main<CL, P, WEIGHT, 1>(a, w, coord, grid, st); break;
+    case 2: rc = cx_scatter_main<CL, P, WEIGHT, 2>(a, w, coord, grid, st); break;
+    default: rc = cx_scatter_main<CL, P, WEIGHT, 3>(a, w, coord, grid, st); break;
     }
-    const int rc = after_launch(WEIGHT ? "to_weight_map (certified, chunked)"
-                                       : "to_map (certified, chunked)");
     if (rc != SO3G_OK) return rc;
     if constexpr (CL == CX_CAR) {
         return cx_scatter_fix<SO3G_COORD_CAR, P, WEIGHT>(a, w, st);

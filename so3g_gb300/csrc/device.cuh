@@ -642,14 +642,15 @@ __device__ __forceinline__ void flush_runs(long long key, long long plane, float
     }
 }
 
-// A kernel's device-side gate: it returns at once when *count > limit (skip)
-// or when *count <= limit (!skip); none when count is NULL.
+// A kernel's device-side gate: it returns at once when more than 1 in `share`
+// of votes[1] are in votes[0] (skip), or when not (!skip); none when votes is
+// NULL.
 struct SkipIf {
-    const unsigned *count = nullptr;
-    unsigned limit = 0;
+    const unsigned long long *votes = nullptr;
+    unsigned share = 0;
     bool skip = false;
     __device__ __forceinline__ bool holds() const {
-        return count && (__ldg(count) > limit) == skip;
+        return votes && (__ldg(votes) * share > __ldg(votes + 1)) == skip;
     }
 };
 

@@ -49,9 +49,10 @@ struct ScatterArgs {
 // The chunked certified to_map / to_weight_map (cert_scatter.cu,
 // cert_weight.cu) over n_seg segments of up to max_len samples of n_det
 // detectors; 1 (nothing launched) where it does not apply.  On SO3G_OK the
-// chunked kernels are launched and skip, on the device, a boresight too
-// rough for them; the caller must then launch the general kernel, which
-// a.gate makes skip in the other case, and free *work (stream-ordered).
+// chunked kernels are launched and skip, on the device, a call whose samples
+// the chunk models would leave to the per-sample path; the caller must then
+// launch the general kernel, which a.gate makes skip in the other case, and
+// free *work (stream-ordered).
 int cert_to_map(int coord, int kind, ScatterArgs &a, int n_det, long long n_seg,
                 long long max_len, cudaStream_t st, void **work);
 int cert_to_weight_map(int coord, int kind, ScatterArgs &a, int n_det, long long n_seg,
