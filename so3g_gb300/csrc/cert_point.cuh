@@ -483,13 +483,11 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
     w[3] = make_float4(0.f, 0.f, __int_as_float(mid), 0.f);
     const CxBore &cb = cxb[j];
     const float E = __ldg(&cb.e), lsb = __ldg(&cb.lsb);
-    // The norm of q(t) q_det: its distance from 1, and from the middle's.
-    float eta, spread;
-    {
+    // The norm of q(t) q_det: its distance from 1.
+    auto norm_off = [&]() {
         const dfl qq = df_dot<4>(qd, qd);
-        eta = __ldg(&cb.eta) + fabsf((qq.hi - 1.f) + qq.lo);
-        spread = 1.01f * __ldg(&cb.spread);
-    }
+        return __ldg(&cb.eta) + fabsf((qq.hi - 1.f) + qq.lo);
+    };
     // (A side's norm may be off by E, which the bilinear form does not cover.)
     const bool covered = __ldg(&cb.part) == 0.f;
     if (!(E < 1e-6f) || (BL && !covered)) return;
@@ -608,11 +606,12 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         lutx = 2.f * 3.1e-10f;
         luty = (HP ? 1.f : 2.f) * 4.7e-10f * zs * rs * rs * rs;
         // The norm N = |alpha|^2 + |beta|^2: the reference's sin(lat) is N
-        // tanh(ln|alpha / beta|), so a sample's N off the middle's by up to
-        // `spread` moves it by spread |tanh|, and the coefficients above, which
+        // tanh(ln|alpha / beta|), so a sample's N off the middle's (by up to
+        // spread) moves it by spread |tanh|, and the coefficients above, which
         // take C^2 for 1 - S^2 (it is N^2 - S^2) and N for 1, are off by up to 5
         // eta / (1 - S^2) of their terms (eta <= 1e-3 here, 1 - S^2 > 0.016).  (A
         // residual moves ln|alpha / beta| by 2 E / C.)
+        const float eta = norm_off(), spread = 1.01f * __ldg(&cb.spread);
         const float ms = mu + 2.2f * E * rs;
         ty += (1.1f * spread * zs + 5.f * eta * ms) * (HP ? 1.f : rs);
         // The spin factors' modulus is (N^2 - S^2) / (1 - S^2), not 1.
@@ -921,7 +920,7 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
             }
             const float ka = cx_gradient<CL>(N0, d32, g0), kb = cx_gradient<CL>(N1, d32, g1);
             const float km = fmaxf(ka, kb) + 1.f;
-            e += aP * (E * (2.1f * gerr + km * (64.f * u + 4.f * eta)) + 16.f * km * km * E * E +
+            e += aP * (E * (2.1f * gerr + km * (64.f * u + 4.f * norm_off())) + 16.f * km * km * E * E +
                        2.f * (km + 4.f) * lsb);
             const float hm = 0.5f * lsb, hd = lsb * s1;
             w[7].z = (g1[0] - g0[0]) * hd;
