@@ -1122,7 +1122,9 @@ __device__ __forceinline__ bool cx_sample(const float4 *w, f32x2 k2, const float
     return ok;
 }
 
-// The residuals of samples t .. t + 3 (t a multiple of 4).
+// The residuals of samples t .. t + 3 (t a multiple of 4, below kCxLen (n_chunks
+// + 1): the lanes of a round without a chunk of their own read on past the last
+// one, where the array is padded, and use nothing of it).
 __device__ __forceinline__ void cx_residuals(const short4 *resid, int t, float (&r)[4][3]) {
     const int4 *p = reinterpret_cast<const int4 *>(resid + t);
     const int4 u = __ldg(p), v = __ldg(p + 1);
@@ -1291,7 +1293,8 @@ inline bool cx_work(CxWork &w, const double *bore, int n_time, long long samples
     const long long n_chunks = (n_time + kCxLen - 1) / kCxLen;
     const long long cap1 = samples / 10 + 4096, cap2 = samples / 96 + 4096;
     const size_t o_res = 256 + sizeof(CxBore) * (size_t)n_chunks;
-    const size_t o_l1 = o_res + sizeof(short4) * (size_t)(n_chunks * kCxLen);
+    // (One chunk of padding: cx_residuals.)
+    const size_t o_l1 = o_res + sizeof(short4) * (size_t)((n_chunks + 1) * kCxLen);
     const size_t o_l2 = o_l1 + sizeof(int2) * (size_t)cap1;
     const size_t bytes = o_l2 + sizeof(int2) * (size_t)cap2;
     if (cudaMallocAsync(&w.mem, bytes, stream) != cudaSuccess) {
