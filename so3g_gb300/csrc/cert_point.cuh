@@ -794,8 +794,8 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         const float y2 = cy2 * icy * s2, y3 = cy3 * icy * s3, y4p = x4.r * icy * s4;
         // Errors: the terms left out, the corrections' float32 roundings and
         // those of the coefficients (12u of their terms), the residual's
-        // second order and quantisation, its gradient's linear form, and
-        // the residual's part that is no turn: it scales q, and X and Y with it
+        // second order and quantisation, its gradient's linear form (which
+        // takes the quaternions for unit ones), and the residual's part that is no turn: it scales q, and X and Y with it
         // (SIN 2, ZEA 1, TAN 2 / cos(theta) times their size).
         const float cor = 1024.f * (fabsf(cx2 * icx) + fabsf(cy2 * icy)) * s2 +
                           32768.f * (fabsf(cx3 * icx) + fabsf(cy3 * icy)) * s3 + 2e-4f;
@@ -803,7 +803,8 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         const float far = fmaxf(fabsf(X0.hi), fabsf(Y0.hi)) + fmaxf(sx, sy);
         const float eb = tx * ai + 12.f * u * cor + 3e-12f * rx * ai +
                          1.2f * xs * far * __ldg(&cb.rho0) * ai +
-                         (lsb > 0.f ? rx * ai * (E * (16.f * E + 2.f * zz + 32.f * u) + 2.f * lsb)
+                         (lsb > 0.f ? rx * ai * (E * (16.f * E + 2.f * zz + 32.f * u + 4.f * norm_off()) +
+                                                 2.f * lsb)
                                     : rx * ai * E);
         if (!(eb < kCxBlPix && (sx * aix + 1.f) < 60.f && (sy * aiy + 1.f) < 60.f)) return;
         w[0] = make_float4(fx0, fy0, fx1, fy1);

@@ -40,17 +40,20 @@ def _scan(boresight):
     q = np.asarray(quat.rotation_xieta(x * DEG, 3. * DEG + 0. * x, 0.2 + 0. * x))
     if boresight == "float32":
         q = q.astype(np.float32).astype(float)
-    elif boresight == "noise":
-        q = q + 1e-8 * rng.standard_normal(q.shape)
+    elif boresight in ("noise", "unit-noise"):
+        q = q + (1e-8 if boresight == "noise" else 2e-8) * rng.standard_normal(q.shape)
+        if boresight == "unit-noise":
+            q /= np.sqrt((q * q).sum(1, keepdims=True))
     return q
 
 
-def _call(proj, boresight):
+def _call(proj, boresight, norm=1.):
     """(engine, map, arguments): a checkerboard of 0.5 arcmin pixels."""
     import torch
     k = np.arange(N_DET)
     r, a = 1. * DEG * np.sqrt((k + .5) / N_DET), 2.4 * k
     dets = np.asarray(quat.rotation_xieta(r * np.cos(a), r * np.sin(a), 0.7 * k))
+    dets = dets * np.sqrt(norm)
     resp = np.ones((N_DET, 2), np.float32)
     args = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (_scan(boresight), dets, resp)]
     ny, nx = 1201, 1502
@@ -63,7 +66,17 @@ def _call(proj, boresight):
 @pytest.mark.parametrize("boresight", ["unit", "float32", "noise", "accelerating"])
 @pytest.mark.parametrize("proj", ["TAN", "ZEA", "SIN"])
 def test_residual_norm(gpulib, proj, boresight):
-    eng, m, args = _call(proj, boresight)
+    _check_mixed(*_call(proj, boresight))
+
+
+@pytest.mark.parametrize("norm", [1.00098, 0.99905])
+@pytest.mark.parametrize("proj", ["TAN", "ZEA", "SIN"])
+def test_detector_norm(gpulib, proj, norm):
+    """The residual's turn, with detector quaternions off unit length."""
+    _check_mixed(*_call(proj, "unit-noise", norm))
+
+
+def _check_mixed(eng, m, args):
     eng.pointing = _abi.POINTING_MIXED
     chunked, general = _both(lambda: eng.from_map(m, *args, None))
     assert float((general != 0).float().mean()) > 0.3
