@@ -287,8 +287,8 @@ class ClockSampler:
 # the signal (4 B read, from_map also 4 B written) and the boresight per
 # detector, so it scales with the samples.
 MEASURED_TRAFFIC_PER_SAMPLE = {
-    "certified": {"to_map": (811.80e6 + 16.89e6) / 2e8,
-                  "from_map": (813.74e6 + 952.03e6) / 2e8},
+    "certified": {"to_map": (811.34e6 + 17.33e6) / 2e8,
+                  "from_map": (813.35e6 + 849.35e6) / 2e8},
     "mixed": {"to_map": (807.045e6 + 13.405e6) / 2e8,
               "from_map": (806.769e6 + 790.061e6) / 2e8},
 }
