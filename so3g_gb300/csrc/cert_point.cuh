@@ -88,7 +88,7 @@ struct __align__(16) CxBore {
     float lsb;             // residuals' unit; 0: none kept (e is negligible)
     float part;            // 1: some samples are not covered (residuals kCxUncovered)
     float rho0;            // max |Re(conj(q) (q - Q))|, the residuals' part that is no turn
-    float pad[2];
+    float q1, qr;          // sizes at the chunk's end: |a1| / 2; |a2| / 4 + |a3| / 8 + |a4| / 16
 };
 
 // The boresight models of a call: per chunk, and the residuals per sample.
@@ -283,13 +283,16 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
         }
     }
     const float lsb = quad && !bad ? E2 * (1.f / 32000.f) : 0.f;
+    const float b1_ = quad ? p1.hi : a1.hi, b2_ = quad ? p2.hi : a2.hi;
+    const float n1 = sqrtf(sum4(b1_ * b1_)), n2 = sqrtf(sum4(b2_ * b2_)),
+                n3 = sqrtf(sum4(a3 * a3)), n4 = sqrtf(sum4(a4 * a4));
     if (chunk < n_chunks && part == 0) {
         float *o = reinterpret_cast<float *>(out + j);
         o[comp] = q0.hi;
         o[4 + comp] = q0.lo;
-        o[8 + comp] = quad ? p1.hi : a1.hi;
+        o[8 + comp] = b1_;
         o[12 + comp] = quad ? p1.lo : a1.lo;
-        o[16 + comp] = quad ? p2.hi : a2.hi;
+        o[16 + comp] = b2_;
         o[20 + comp] = quad ? 0.f : a3;
         o[24 + comp] = quad ? 0.f : a4;
         if (comp == 0) {
@@ -298,6 +301,9 @@ __global__ void __launch_bounds__(128) k_cx_bore(const double *bore, int n_time,
             out[j].spread = bad ? 1.f : spread * 1.00001f + 1e-14f;
             out[j].lsb = lsb;
             if (!(lsb > 0.f)) out[j].rho0 = out[j].e;
+            // (1.001: the detector quaternions' norm.)
+            out[j].q1 = 1.001f * 0.5f * n1;
+            out[j].qr = 1.001f * (0.25f * n2 + (quad ? 0.f : 0.125f * n3 + 0.0625f * n4));
             out[j].part = c0 > k0 || c1 < k1 ? 1.f : 0.f;
         }
     }
@@ -399,6 +405,36 @@ __device__ __forceinline__ float cx_tail_log(const CxTail &t) {
 __device__ __forceinline__ float cx_tail_exp(const CxTail &t) {
     const float x2 = t.X * t.X;
     return 0.5f * t.t2 + (1.f / 6.f) * t.t3 + (1.f / 24.f) * t.t4 + (1.f / 100.f) * x2 * x2 * t.X;
+}
+
+// Size of the terms of order >= m of a zenithal projection's factor e(u)
+// (cx_setup), m = 5 (BL) or 4, at the chunk's end, from the sizes a1 .. a4 of
+// alpha's relative coefficients.  Nothing is taken to fall off from one order
+// to the next: a scan may accelerate (a2 against a1^2), and the quartic of a
+// short last chunk carries noise in every order.
+// SIN: e = alpha / alpha_0.  ZEA: exp(i theta), m1 .. m4 theta's sizes.
+// TAN: alpha / alpha_0 times G = 1 / (1 + x), x = f (|alpha / alpha_0|^2 - 1).
+template <bool BL>
+__device__ __forceinline__ float cx_rest_zea(float m1, float m2, float m3, float m4, float tail) {
+    const float r5 = cx_tail_exp(cx_tail(m1, m2, m3, m4)) + 1.1f * tail;
+    if (BL) return r5;
+    return r5 + m4 + m1 * m3 + 0.5f * m2 * m2 + 0.5f * m1 * m1 * m2 +
+           (1.f / 24.f) * m1 * m1 * m1 * m1;
+}
+template <bool BL>
+__device__ __forceinline__ float cx_rest_tan(float f, float a1, float a2, float a3, float a4) {
+    const float y1 = 2.f * f * a1, y2 = f * (2.f * a2 + a1 * a1), y3 = 2.f * f * (a3 + a1 * a2),
+                y4 = f * (2.f * a4 + 2.f * a1 * a3 + a2 * a2);
+    const float y5 = 2.f * f * (a4 * (a1 + a2 + a3) + a2 * a3) + f * (a3 * a3 + a4 * a4);
+    const CxTail t = cx_tail(y1, y2, y3, y4);
+    const float Y = t.X + y5, Y2 = Y * Y;
+    const float g1 = y1, g2 = y2 + y1 * y1, g3 = y3 + 2.f * y1 * y2 + y1 * y1 * y1,
+                g4 = y4 + 2.f * y1 * y3 + y2 * y2 + 3.f * y1 * y1 * y2 + y1 * y1 * y1 * y1;
+    const float g5 = y5 * (1.f + 3.f * Y) + t.t2 + t.t3 + t.t4 + 1.3f * Y2 * Y2 * Y;
+    const float r5 = g5 * (1.f + a1 + a2 + a3 + a4) + a4 * (g1 + g2 + g3 + g4) +
+                     a3 * (g2 + g3 + g4) + a2 * (g3 + g4) + a1 * g4;
+    if (BL) return r5;
+    return r5 + a4 + a3 * g1 + a2 * g2 + a1 * g3 + g4;
 }
 
 // Gradient of phi with respect to a rotation rho of the boresight (q (1 +
@@ -523,10 +559,23 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
     const float d32[4] = {qd[0].hi, qd[1].hi, qd[2].hi, qd[3].hi};
     const float A[4] = {qa.hi, qb.hi, qc.hi, qe.hi};
     float A1[4], A2[4], A3[4], A4[4];
-    cx_qmul(__ldg(&cb.a1_hi), d32, A1);
+    dfl B1[4];   // BL: A1 in double-float
+    if constexpr (BL) {
+        const float4 h = __ldg(&cb.a1_hi), l = __ldg(&cb.a1_lo);
+        const dfl q[4] = {{h.x, l.x}, {h.y, l.y}, {h.z, l.z}, {h.w, l.w}};
+        df_qmul(q, qd, B1[0], B1[1], B1[2], B1[3]);
+#pragma unroll
+        for (int c = 0; c < 4; c++) A1[c] = B1[c].hi;
+    } else {
+        cx_qmul(__ldg(&cb.a1_hi), d32, A1);
+    }
     cx_qmul(__ldg(&cb.a2), d32, A2);
     cx_qmul(__ldg(&cb.a3), d32, A3);
     cx_qmul(__ldg(&cb.a4), d32, A4);
+    // Their sizes at the chunk's end: the coefficients' float32 errors go with
+    // the quaternions', not with alpha's or beta's (6u each: the operands' roundings
+    // and the product's).
+    const float Q1 = __ldg(&cb.q1), Qr = __ldg(&cb.qr);
     const float al2 = A[0] * A[0] + A[3] * A[3], be2 = A[1] * A[1] + A[2] * A[2];
     const float nq2 = d32[0] * d32[0] + d32[1] * d32[1] + d32[2] * d32[2] + d32[3] * d32[3];
     if (!(fabsf(al2 + be2 - 1.f) < 1e-3f && fabsf(nq2 - 1.f) < 1e-3f && al2 > 0.004f)) return;
@@ -548,7 +597,11 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
     float lutx = 0.f, luty = 0.f;    // the tables' errors at both ends
     float zz;                        // |z1|^2 of alpha and beta
     float gerr;                      // gradient of phi: error of its linear form
-    float mod = 0.f;                 // spin factors' modulus: change over the chunk (relative)
+    float es;                        // spin factors (relative): change of the modulus over the
+                                     // chunk, float32 errors of phi2 .. phi4
+    float big;                       // size of the terms that X, Y's coefficients are sums of
+    float curv = 0.f;                // BL: curvature of the pixel's gradient
+    float sx2 = 0.f;                 // BL: terms of X, Y's coefficients of order >= 2
     cf x4{0.f, 0.f};                 // BL: the u^4 coefficient of Y - i X,
     float xs = 2.f;                  // and X, Y's change with the norm of q (relative)
     if constexpr (CL == CX_CAR) {
@@ -568,6 +621,9 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         phi3 = 2.f * (la.l3.i + lb.l3.i);
         phi4 = 2.f * (la.l4.i + lb.l4.i);
         zz = 4.f * (ta.X * ta.X + tb.X * tb.X);
+        // 2 x 9u of each of la's and lb's (6u, and 3u of the division).
+        es = 18.f * u * Qr * (ra + rb);
+        big = 0.3f * (Q1 + Qr) * (ra + rb);   // (9u of Q1 + Qr)
         cx1 = la.l1.i - lb.l1.i;
         cx2 = la.l2.i - lb.l2.i;
         cx3 = la.l3.i - lb.l3.i;
@@ -580,9 +636,10 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
                     mu4 = 0.0625f * fabsf(la.l4.r - lb.l4.r) + tail;
         const float mu = mu1 + mu2 + mu3 + mu4;
         // kappa = S / v, |v| = C / 2: |kappa''| / 8 with |(1/v)'| <= |z1a| +
-        // |z1b|, |S'| <= C^2 |m1|, |S''| <= 2 C^2 (m1^2 + |m2|).
+        // |z1b|, |(1/v)''| <= (...)^2 + 2 |l2a + l2b|, |S'| <= C^2 |m1|, |S''| <=
+        // 2 C^2 (m1^2 + |m2|).
         const float zs1 = 2.f * (ta.X + tb.X);
-        gerr = 0.3f * fabsf(S) * rsqrtf(C2) * zs1 * zs1 +
+        gerr = fabsf(S) * rsqrtf(C2) * (0.3f * zs1 * zs1 + 0.75f * cf_abs(la.l2 + lb.l2)) +
                C * fabsf(m1) * (0.6f * zs1 + 0.6f * fabsf(m1)) + 0.6f * C * fabsf(m2);
         // Order >= 4: m's own, those of m^2 / 2 and m^3 / 6 (derivatives at
         // most 2 and 4), and the fourth derivative's (at most 10).
@@ -615,7 +672,7 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         const float ms = mu + 2.2f * E * rs;
         ty += (1.1f * spread * zs + 5.f * eta * ms) * (HP ? 1.f : rs);
         // The spin factors' modulus is (N^2 - S^2) / (1 - S^2), not 1.
-        mod = rs * rs * (2.2f * spread + 5.f * eta * zs * ms);
+        es += 1.1f * rs * rs * (2.2f * spread + 5.f * eta * zs * ms);
         // The longitude stays inside (-pi, pi) over the chunk (a HEALPix pixel
         // takes it modulo 2 pi).
         if (!HP && !(fabsf(X0.hi) + 1.05f * (ta.X + tb.X) + rx * E + 1e-6f < 3.1415f)) return;
@@ -626,9 +683,11 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         phi4 = 4.f * la.l4.i;
         zz = 4.f * ta.X * ta.X;
         if (!(al2 > 0.25f)) return;
+        es = 36.f * u * Qr * ra;
+        big = 4.f * (ta.X + Q1 + Qr);
         // kappa = -2 conj(beta) / alpha: |kappa''| / 8.
         gerr = 0.6f * ra * (cf_abs(cf{A2[2], A2[1]}) + 2.f * ta.X * cf_abs(cf{A1[2], A1[1]}) +
-                            4.f * ta.X * ta.X);
+                            4.f * ta.X * ta.X + cf_abs(la.l2));
         // Y - i X = 2 g(n_0) alpha_0 e(u) conj(beta), e = (alpha / alpha_0)
         // g(n) / g(n_0): SIN alpha / alpha_0, ZEA exp(i Im la), TAN (alpha /
         // alpha_0) / (1 + x), x = 2 (n - n_0) / (2 n_0 - 1), n = n_0 exp(2 Re la).
@@ -636,6 +695,10 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         const cf z2 = cf{A2[0], A2[3]} * inv_a, z3 = cf{A3[0], A3[3]} * inv_a;
         cf e1, e2, e3;
         float g = 2.f, h = 1.1f * ta.X;   // h: size of e - 1 at the chunk's end
+        float ft = 0.f;                   // TAN: f
+        const float s1_ = 0.5f * cf_abs(z1), s2_ = 0.25f * cf_abs(z2), s3_ = 0.125f * cf_abs(z3),
+                    s4_ = 0.0625f * cf_abs(cf{A4[0], A4[3]} * inv_a);
+        float rest = BL ? 0.f : s4_;      // e's terms left out
         rx = 2.2f;
         if (coord == SO3G_COORD_TAN) {
             const float ct = 2.f * al2 - 1.f;
@@ -651,6 +714,8 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
             g *= ic;
             xs = 2.f * ic;
             h += 2.4f * f * ta.X;
+            ft = f;
+            rest = cx_rest_tan<BL>(f, s1_, s2_, s3_, s4_);
             // (2 ic^2 for a turn, 2 ic^2 sin(theta) for a change of norm.)
             rx = 2.9f * ic * ic;
         } else if (coord == SO3G_COORD_ZEA) {
@@ -659,6 +724,8 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
             e2 = cf{-0.5f * t1 * t1, t2};
             e3 = cf{-t1 * t2, t3 - (1.f / 6.f) * t1 * t1 * t1};
             g *= rsqrtf(al2);
+            rest = cx_rest_zea<BL>(0.5f * fabsf(t1), 0.25f * fabsf(t2), 0.125f * fabsf(t3),
+                                   0.0625f * fabsf(la.l4.i), tail);
             xs = 1.f;
             rx = 2.4f * ia;
         } else {
@@ -678,12 +745,12 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         cx1 = -p1.i;
         cx2 = -p2.i;
         cx3 = -p3.i;
-        // Order >= 4 of e times beta: with bk = |b_k| / 2^k and e's terms of
-        // order n below 2 h^n (h covers alpha's, the exponential's and TAN's
-        // series at the chunk's end).
+        // The terms left out of e times conj(beta) (order >= 4, BL: >= 5), with the
+        // sizes kn = |b_n| / 2^n, dn = |e_n| / 2^n.
+        const float d1 = 0.5f * cf_abs(e1), d2 = 0.25f * cf_abs(e2), d3 = 0.125f * cf_abs(e3);
         const float k0 = cf_abs(b0), k1 = 0.5f * cf_abs(b1), k2 = 0.25f * cf_abs(b2),
                     k3 = 0.125f * cf_abs(b3), k4 = 0.0625f * cf_abs(cf{A4[2], A4[1]});
-        const float h2 = h * h;
+        const float ks = k1 + k2 + k3 + k4;
         if constexpr (BL) {
             // (One order more.)
             const cf b4{A4[2], -A4[1]};
@@ -708,11 +775,19 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
                 e4 = cf{A4[0], A4[3]} * inv_a;
             }
             x4 = s * (b4 + e1 * b3 + e2 * b2 + e3 * b1 + e4 * b0);
-            tx = ty = g * 5.f * h * (k0 * h2 * h2 + k1 * h2 * h + k2 * h2 + k3 * h + 1.2f * k4) *
-                          1.2f + 1e-13f;
+            const float d4 = 0.0625f * cf_abs(e4);
+            tx = ty = 1.2f * g * (rest * (k0 + ks) + d1 * k4 + d2 * (k3 + k4) +
+                                  d3 * (k2 + k3 + k4) + d4 * ks) + 1e-13f;
+            // (b_n and e_n: the quaternions' 6u, of A1 u, and 3u of a division; 24u
+            // of the products' terms.)
+            sx2 = g * (8.f * Qr * (1.f + 2.f * (1.f + ft) * (k0 + k1)) +
+                       2.5f * (1.f + 2.f * ft) * Q1 * k1 +
+                       24.f * (d1 * (ks + Q1) + (d2 + d3 + d4) * (k0 + ks)));
+            const float zn = 2.f * s1_ * (1.f + 2.f * ft) + 2.f * k1;
+            curv = 1.5f * (zn * zn + 4.f * s2_ * (1.f + ft) + 4.f * k2);
         } else {
-            tx = ty = g * (4.f * (k0 * h2 * h2 + k1 * h2 * h + k2 * h2 + k3 * h) + 1.2f * k4) *
-                          1.2f + 1e-12f;
+            tx = ty = 1.2f * g * (rest * (k0 + ks) + k4 + d1 * (k3 + k4) + d2 * (ks - k1) +
+                                  d3 * ks) + 1e-12f;
         }
     }
     // Pixel coordinates: the coefficients' float32 errors (24u of the terms'
@@ -722,8 +797,8 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
     const float aix = fabsf(icx), aiy = fabsf(icy);
     const float sx = 0.5f * fabsf(cx1) + 0.25f * fabsf(cx2) + 0.125f * fabsf(cx3);
     const float sy = 0.5f * fabsf(cy1) + 0.25f * fabsf(cy2) + 0.125f * fabsf(cy3);
-    const float big = CL == CX_CAR ? ta.X * 4.f + sx + sy + zz
-                                   : 4.f * (ta.X + 0.5f * cf_abs(cf{A1[2], A1[1]})) * (1.f + rx);
+    if (CL == CX_CAR) big = fmaxf(big, ta.X * 4.f + sx + sy + zz);
+    else big *= 1.f + rx;
     float ex = (tx + lutx + rx * E + 32.f * u * (sx + big)) * aix;
     float ey = (ty + luty + ry * E + 32.f * u * (sy + big)) * aiy;
     int xb = 0, yb = 0;
@@ -755,12 +830,7 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         // X', Y' at the middle in double-float: Y' - i X' = s b1 + e1 (Y0 - i
         // X0), s = 2 g alpha_0, b1 = conj(beta_1), e1 = i Im z1 (ZEA), z1 (SIN)
         // or z1 - 4 n Re(z1) / (2n - 1) (TAN), z1 = alpha_1 / alpha_0.
-        dfl p, r, s, t;
-        {
-            const float4 h = __ldg(&cb.a1_hi), l = __ldg(&cb.a1_lo);
-            const dfl q[4] = {{h.x, l.x}, {h.y, l.y}, {h.z, l.z}, {h.w, l.w}};
-            df_qmul(q, qd, p, r, s, t);
-        }
+        const dfl p = B1[0], r = B1[1], s = B1[2], t = B1[3];
         const dfl n = df_dot<2>({qa, qe}, {qa, qe}), rn = df_recip(n);
         const dfl ei = df_mul(df_dot<2>({t, p}, {qa, df_neg(qe)}), rn);
         dfl er = df_mul(df_dot<2>({p, t}, {qa, qe}), rn), G{2.f, 0.f};
@@ -793,7 +863,7 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         const float x2 = cx2 * icx * s2, x3 = cx3 * icx * s3, x4p = -x4.i * icx * s4;
         const float y2 = cy2 * icy * s2, y3 = cy3 * icy * s3, y4p = x4.r * icy * s4;
         // Errors: the terms left out, the corrections' float32 roundings and
-        // those of the coefficients (12u of their terms), the residual's
+        // those of the coefficients (sx2), the residual's
         // second order and quantisation, its gradient's linear form (which
         // takes the quaternions for unit ones), and the residual's part that is no turn: it scales q, and X and Y with it
         // (SIN 2, ZEA 1, TAN 2 / cos(theta) times their size).
@@ -801,9 +871,9 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
                           32768.f * (fabsf(cx3 * icx) + fabsf(cy3 * icy)) * s3 + 2e-4f;
         const float ai = fmaxf(aix, aiy);
         const float far = fmaxf(fabsf(X0.hi), fabsf(Y0.hi)) + fmaxf(sx, sy);
-        const float eb = tx * ai + 12.f * u * cor + 3e-12f * rx * ai +
+        const float eb = tx * ai + u * (4.f * cor + sx2 * ai) + 3e-12f * rx * ai +
                          1.2f * xs * far * __ldg(&cb.rho0) * ai +
-                         (lsb > 0.f ? rx * ai * (E * (16.f * E + 2.f * zz + 32.f * u + 4.f * norm_off()) +
+                         (lsb > 0.f ? rx * ai * (E * (16.f * E + curv + 32.f * u + 4.f * norm_off()) +
                                                  2.f * lsb)
                                     : rx * ai * E);
         if (!(eb < kCxBlPix && (sx * aix + 1.f) < 60.f && (sy * aiy + 1.f) < 60.f)) return;
@@ -898,15 +968,15 @@ __device__ __forceinline__ void cx_setup(const Args &a, const CxBore *cxb, int c
         w[7] = make_float4(o[0][6], o[1][6], 0.f, 0.f);
         // e: the double-float error and the reference's roundings (kEpsPf;
         // phi1's is of the same size), the terms left out, the modulus'
-        // change, the float32 errors of phi2 (16u |z1|^2), phi3,
-        // phi4 and of the products, the correction's roundings (3u of its
+        // change and the float32 errors of phi2, phi3 and phi4 (es, and 16u |z1|^2)
+        // and of the products, the correction's roundings (3u of its
         // terms), and the boresight's distance from Q.
         const float h1 = 0.5f * fabsf(p1), h2 = 0.25f * fabsf(phi2) + u * zz,
                     h3 = 0.125f * fabsf(phi3) + 8.f * u * zz, h4 = 0.0625f * fabsf(phi4) + 8.f * u * zz;
         const CxTail tp = cx_tail(h1, h2, h3, h4);
         const float Df = D.hi;
         e = 1.2f * (cx_tail_exp(tp) + 4.f * tail) +
-            kEpsPf * fmaxf(1.f, 0.25f / Df) * (1.f + h1) + 1.1f * mod +
+            kEpsPf * fmaxf(1.f, 0.25f / Df) * (1.f + h1) + es +
             u * (3.f * h1 * h1 + 8.f * h2 + 4.f * zz + 16.f * (h3 + h4 + h1 * (h2 + h1 * h1)));
         e = e * fmaxf(aP, 1e-3f) + 3.f * u * 18.f * gr;
         if (lsb > 0.f) {

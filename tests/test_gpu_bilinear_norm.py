@@ -47,8 +47,8 @@ def _scan(boresight):
     return q
 
 
-def _call(proj, boresight, norm=1.):
-    """(engine, map, arguments): a checkerboard of 0.5 arcmin pixels."""
+def _call(proj, boresight, norm=1., res=.5):
+    """(engine, map, arguments): a checkerboard of `res` arcmin pixels."""
     import torch
     k = np.arange(N_DET)
     r, a = 1. * DEG * np.sqrt((k + .5) / N_DET), 2.4 * k
@@ -56,9 +56,9 @@ def _call(proj, boresight, norm=1.):
     dets = dets * np.sqrt(norm)
     resp = np.ones((N_DET, 2), np.float32)
     args = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (_scan(boresight), dets, resp)]
-    ny, nx = 1201, 1502
+    ny, nx = (1201, 1502) if res >= .5 else (2001, 2502)
     eng = getattr(so3g, "ProjEng_%s_T_NonTiled_Bilinear" % proj)(
-        (ny, nx, .5 * synth.ARCMIN, -.5 * synth.ARCMIN, ny / 2. + .5, nx / 2. + .5))
+        (ny, nx, res * synth.ARCMIN, -res * synth.ARCMIN, ny / 2. + .5, nx / 2. + .5))
     yx = torch.arange(ny, device="cuda")[:, None] + torch.arange(nx, device="cuda")
     return eng, (1. - 2. * (yx % 2)).double()[None].contiguous(), args
 
@@ -74,6 +74,23 @@ def test_residual_norm(gpulib, proj, boresight):
 def test_detector_norm(gpulib, proj, norm):
     """The residual's turn, with detector quaternions off unit length."""
     _check_mixed(*_call(proj, "unit-noise", norm))
+
+
+@pytest.mark.parametrize("seed", [1, 2, 3])
+@pytest.mark.parametrize("proj", ["TAN", "ZEA", "SIN"])
+def test_short_last_chunk(gpulib, proj, seed):
+    """A last chunk of one sample, its model's other samples the chunk before's,
+    with pointing noise: a polynomial through the one sample it is used at,
+    with noise in every order."""
+    import torch
+    n = 64 * 200 + 1
+    s = np.abs((np.arange(n) - n + 700) / 200. * 1.4 % 18. - 9.) - 4.5
+    q = np.asarray(quat.rotation_xieta(s * DEG, 1. * DEG + 0. * s, 0.2 + 0. * s))
+    q[-65:] += 3e-8 * np.random.default_rng(seed).standard_normal((65, 4))
+    q /= np.sqrt((q * q).sum(1, keepdims=True))
+    eng, m, args = _call(proj, "unit", res=.3)
+    args[0] = torch.from_numpy(np.ascontiguousarray(q)).cuda()
+    _check_mixed(eng, m, args)
 
 
 def _check_mixed(eng, m, args):
