@@ -13,7 +13,7 @@
 // of the issue slots at 24 warps per SM).  CAR TQU 3 x 2000 x 2000, 1000 det x
 // 1M samples: 30.9 -> 8.4 ms, and with the steps that two quantities or two
 // samples share as f32x2 instructions 7.7 ms; with models for the longer side
-// of the turn-arounds 7.2 ms (of which 0.9 ms the fallback).
+// of the turn-arounds 7.3 ms (of which 0.93 ms the fallback).
 
 #include "cert_point.cuh"
 #include "cert_map.cuh"

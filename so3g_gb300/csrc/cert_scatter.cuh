@@ -17,9 +17,9 @@
 // the per-sample path ~910), then by the L2 atomic units.  CAR TQU 3 x 2000 x
 // 2000, 1000 det x 1M samples: to_map 26.1 -> 8.3 ms, with f32x2 instructions
 // for the coordinates, the spin factors and the runs' sums 8.0 ms, with models
-// for the longer side of the turn-arounds 7.9 ms (of which 0.74 ms the
-// fallback), to_weight_map of 500 x 500k 7.4 -> 2.8 ms; HEALPix nside 1024, 400
-// det x 500k, to_map + from_map 14.8 -> 5.65 ms.
+// for the longer side of the turn-arounds 7.9 ms, with the bounds on accelerating
+// scans 8.0 ms (of which 0.78 ms the fallback), to_weight_map of 500 x 500k 7.4 ->
+// 2.8 ms; HEALPix nside 1024, 400 det x 500k, to_map + from_map 14.8 -> 5.8 ms.
 #pragma once
 
 #include <algorithm>
